@@ -75,7 +75,7 @@ __host__ __device__ inline BLayout blayout(uint32_t nq, uint32_t nchain, uint32_
   L.off_sum = o = align_up(o, 16);
   o += nq * 8;  // per query: 1-group sum
   L.off_cnt = o;
-  o += nq * 8;  // per query: kept rows
+  o += nq * 4;  // per query: kept rows
   L.off_toff = o;
   o += nq * 4;  // per query: first slot of its shared group table, or BT_NOTABLE
   L.off_bar = o = align_up(o, 8);
@@ -88,7 +88,7 @@ __host__ __device__ inline BLayout blayout(uint32_t nq, uint32_t nchain, uint32_
   o += align_up(nchain * 2, 16);
   L.off_conj = o;
   o += nconj * 4;
-  L.off_stab = o = align_up(o, 16);  // 64-bit atomics: 8-byte aligned at least
+  L.off_stab = o = align_up(o, 16);
   o += nstab * 8;
   L.off_buf = o = align_up(o, 16);
   o += nw * L.buf * 4;
@@ -116,9 +116,10 @@ struct BCtx {
   const uint32_t *sdim;
   const uint32_t *toff;
   unsigned long long *out;
-  unsigned long long *qsum;  // per query: 1-group sum (this CTA)
-  unsigned long long *qcnt;  // per query: kept rows (this CTA)
-  unsigned long long *stab;  // shared group tables
+  uint32_t *qsum;   // per query: 1-group sum (this CTA), a pair of halves (shared_add64)
+  uint32_t *qcnt;   // per query: kept rows (this CTA; below 2^31 as the table's rows are)
+  uint32_t *stab;   // shared group tables: the sums' low halves, then (nstab on) their high halves
+  uint32_t nstab;
 };
 
 // A predicated 32-bit read-only load: 0 where pred is false.  Written out so
@@ -147,17 +148,17 @@ __device__ __forceinline__ void b_accumulate(const BCtx &C, uint32_t q, const ui
 #pragma unroll
     for (int j = 0; j < R; ++j) v += keep[j] ? x[j] : 0;
     const uint64_t s = peer_sum64(0xffffffffu, v);
-    if (lane == 0 && s) atomicAdd(&C.qsum[q], (unsigned long long)s);
+    if (lane == 0 && s) shared_add64(&C.qsum[2 * q], &C.qsum[2 * q + 1], s);
   } else {
     const uint32_t t = C.toff[q];
 #pragma unroll
     for (int j = 0; j < R; ++j)
       if (keep[j]) {
-        if (t != BT_NOTABLE) atomicAdd(&C.stab[t + g[j]], (unsigned long long)x[j]);
+        if (t != BT_NOTABLE) shared_add64(&C.stab[t + g[j]], &C.stab[C.nstab + t + g[j]], x[j]);
         else atomicAdd(&C.out[d[2] + g[j]], (unsigned long long)x[j]);
       }
   }
-  if (lane == 0 && kept) atomicAdd(&C.qcnt[q], (unsigned long long)kept);
+  if (lane == 0 && kept) atomicAdd(&C.qcnt[q], kept);
 }
 
 // Query q's op on R rows per lane (act: the lane has the row; unc: the row
@@ -378,16 +379,16 @@ struct BDrain {
 #pragma unroll
       for (int j = 0; j < R; ++j) sv += keep[j] ? x[j] : 0;
       const uint64_t tot = peer_sum64(0xffffffffu, sv);
-      if (lane == 0 && tot) atomicAdd(&C.qsum[q], (unsigned long long)tot);
+      if (lane == 0 && tot) shared_add64(&C.qsum[2 * q], &C.qsum[2 * q + 1], tot);
     } else {
 #pragma unroll
       for (int j = 0; j < R; ++j)
         if (keep[j]) {
-          if (toff != BT_NOTABLE) atomicAdd(&C.stab[toff + g[j]], (unsigned long long)x[j]);
+          if (toff != BT_NOTABLE) shared_add64(&C.stab[toff + g[j]], &C.stab[C.nstab + toff + g[j]], x[j]);
           else atomicAdd(&C.out[obase + g[j]], (unsigned long long)x[j]);
         }
     }
-    if (lane == 0 && kept) atomicAdd(&C.qcnt[q], (unsigned long long)kept);
+    if (lane == 0 && kept) atomicAdd(&C.qcnt[q], kept);
   }
 };
 
@@ -570,21 +571,21 @@ batch_scan_kernel(const BatchHdr *__restrict__ H, const __grid_constant__ BParam
   unsigned long long *scol = reinterpret_cast<unsigned long long *>(smem + L.off_src);
   unsigned long long *sfk = scol + BS_MAX;
   uint32_t *sdim = reinterpret_cast<uint32_t *>(sfk + BS_MAX), *swid = sdim + BS_MAX;
-  unsigned long long *qsum = reinterpret_cast<unsigned long long *>(smem + L.off_sum);
-  unsigned long long *qcnt = reinterpret_cast<unsigned long long *>(smem + L.off_cnt);
+  uint32_t *qsum = reinterpret_cast<uint32_t *>(smem + L.off_sum);
+  uint32_t *qcnt = reinterpret_cast<uint32_t *>(smem + L.off_cnt);
   uint32_t *toff = reinterpret_cast<uint32_t *>(smem + L.off_toff);
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + L.off_bar), *empty = full + P.S;
   uint32_t *qctr = reinterpret_cast<uint32_t *>(smem + L.off_ctr), *abort_ = qctr + P.S;
   uint8_t *order = smem + L.off_order;
   uint16_t *chain = reinterpret_cast<uint16_t *>(smem + L.off_chain);
   uint32_t *conj = reinterpret_cast<uint32_t *>(smem + L.off_conj);
-  unsigned long long *stab = reinterpret_cast<unsigned long long *>(smem + L.off_stab);
+  uint32_t *stab = reinterpret_cast<uint32_t *>(smem + L.off_stab);
   uint32_t *wbuf = reinterpret_cast<uint32_t *>(smem + L.off_buf) + warp * L.buf;
   uint32_t *stages = reinterpret_cast<uint32_t *>(smem + L.off_stage);
 
   for (uint32_t i = tid; i < P.nq * BQD_WORDS; i += blockDim.x) Qd[i] = H->Qd[i];
-  for (uint32_t i = tid; i < P.nq; i += blockDim.x) qsum[i] = 0, qcnt[i] = 0, toff[i] = H->toff[i];
-  for (uint32_t i = tid; i < P.nstab; i += blockDim.x) stab[i] = 0;
+  for (uint32_t i = tid; i < P.nq; i += blockDim.x) qsum[2 * i] = qsum[2 * i + 1] = 0, qcnt[i] = 0, toff[i] = H->toff[i];
+  for (uint32_t i = tid; i < 2 * P.nstab; i += blockDim.x) stab[i] = 0;
   for (uint32_t i = tid; i < P.nchain; i += blockDim.x) chain[i] = H->chain[i];
   for (uint32_t i = tid; i < P.nconj; i += blockDim.x) conj[i] = H->conj[i];
   for (uint32_t i = tid; i < P.nq; i += blockDim.x) order[i] = H->order[i];
@@ -614,6 +615,7 @@ batch_scan_kernel(const BatchHdr *__restrict__ H, const __grid_constant__ BParam
   C.qsum = qsum;
   C.qcnt = qcnt;
   C.stab = stab;
+  C.nstab = P.nstab;
 
   const uint64_t ntiles = (P.nwords + T - 1) / T;
   // tiles of this CTA (fewer than 2^32: a table has fewer than 2^31 rows)
@@ -700,16 +702,19 @@ batch_scan_kernel(const BatchHdr *__restrict__ H, const __grid_constant__ BParam
   if (*(volatile uint32_t *)abort_) return;
   for (uint32_t q = tid; q < P.nq; q += blockDim.x) {
     const uint32_t *d = Qd + q * BQD_WORDS;
-    if (qsum[q]) atomicAdd(&out[d[2]], qsum[q]);
-    if (qcnt[q]) atomicAdd(&nqual[d[3]], qcnt[q]);
+    const unsigned long long v = qsum[2 * q] | (unsigned long long)qsum[2 * q + 1] << 32;
+    if (v) atomicAdd(&out[d[2]], v);
+    if (qcnt[q]) atomicAdd(&nqual[d[3]], (unsigned long long)qcnt[q]);
   }
   // the shared group tables, one warp per query
   for (uint32_t q = warp; q < P.nq; q += nw) {
     const uint32_t t = toff[q];
     if (t == BT_NOTABLE) continue;
     const uint32_t *d = Qd + q * BQD_WORDS;
-    for (uint32_t g = lane; g < d[1]; g += 32)
-      if (stab[t + g]) atomicAdd(&out[d[2] + g], stab[t + g]);
+    for (uint32_t g = lane; g < d[1]; g += 32) {
+      const unsigned long long v = stab[t + g] | (unsigned long long)stab[P.nstab + t + g] << 32;
+      if (v) atomicAdd(&out[d[2] + g], v);
+    }
   }
 }
 
@@ -773,10 +778,10 @@ static mb_status launch_bs(const BatchHdr &h, const BatchHdr *dh, const BatchCfg
   P.wait_tries = c.wait_tries ? c.wait_tries : (1u << 20);
   P.skip_stage0 = c.skip_stage0;
   P.L = blayout(h.nq, h.nchain, h.nconj, h.nu, c.stages, 32 * V, h.nstab, c.warps, c.buf);
-  // the 64-bit areas (sums, counts, group tables, mbarriers) must be 8-byte
-  // aligned, the stage 128-byte aligned (tensor copies): refuse a layout that
+  // the 64-bit areas (mbarriers, source addresses) must be 8-byte aligned, the
+  // 32-bit atomics' areas 4-byte, the stage 128-byte aligned (tensor copies): refuse a layout that
   // is not, rather than launch it
-  if ((P.L.off_sum | P.L.off_cnt | P.L.off_stab | P.L.off_bar | P.L.off_src) & 7u || (P.L.off_stage & 127u) ||
+  if ((P.L.off_bar | P.L.off_src) & 7u || ((P.L.off_sum | P.L.off_cnt | P.L.off_stab) & 3u) || (P.L.off_stage & 127u) ||
       (P.L.off_buf & 15u) || (P.L.off_conj & 3u) || (P.L.off_toff & 3u) || (P.L.off_ctr & 3u))
     return fail(MB_ERR_INVALID, "batch: shared-memory layout misaligned");
   const DevInfo &di = dev_info();

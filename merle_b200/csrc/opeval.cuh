@@ -105,9 +105,25 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
 // the match.
 constexpr uint32_t GRP_DIRECT_MIN = 2;
 
-// Per-CTA group-by state in shared memory.
+// A 64-bit sum in shared memory kept as two 32-bit halves, `lo` and `hi`: the
+// hardware adds 32-bit words in shared memory but has no 64-bit add there (a
+// 64-bit atomicAdd becomes a compare-and-swap loop that retries per colliding
+// lane).  The carry out of the low half joins the high half's addend, which
+// is zero for almost every 32-bit value of either sign (a negative value's
+// high half is -1 and its low half nearly always carries), so a row costs
+// one 32-bit atomic.  The pair is exact mod 2^64 once every add has finished.
+// Measured at 600M rows on the 64-query selectivity-spanning mix: one launch
+// per query 104.2 -> 102.2 ms, the batched scan 36.6 -> 35.5 ms.
+__device__ __forceinline__ void shared_add64(uint32_t *lo, uint32_t *hi, uint64_t v) {
+  const uint32_t vl = (uint32_t)v, old = atomicAdd(lo, vl);
+  const uint32_t vh = (uint32_t)(v >> 32) + (old + vl < old ? 1u : 0u);
+  if (vh) atomicAdd(hi, vh);
+}
+
+// Per-CTA group-by state in shared memory: the sums as two arrays of 32-bit
+// halves (shared_add64).
 struct GrpCtx {
-  unsigned long long *table;  // GS_SHARED: nr_grp sums; GS_HASH: hash sums
+  uint32_t *lo, *hi;          // GS_SHARED: nr_grp sums; GS_HASH: hash sums
   uint32_t *keys;             // GS_HASH: keys (HASH_EMPTY = free)
   uint32_t hcap;              // GS_HASH: capacity (power of two)
   bool direct;                // GS_SHARED / GS_GLOBAL: one atomic per row (nr_grp >= GRP_DIRECT_MIN)
@@ -120,7 +136,7 @@ __device__ __forceinline__ void hash_add(const GrpCtx &G, uint32_t grp, uint64_t
     uint32_t k = G.keys[h];
     if (k == HASH_EMPTY) k = atomicCAS(&G.keys[h], HASH_EMPTY, grp);
     if (k == HASH_EMPTY || k == grp) {
-      atomicAdd(&G.table[h], (unsigned long long)s);
+      shared_add64(&G.lo[h], &G.hi[h], s);
       return;
     }
     h = (h + 1) & (G.hcap - 1);
@@ -138,7 +154,10 @@ __device__ __forceinline__ void aggregate(const GrpCtx &G, bool kept, uint32_t g
     return;
   }
   if ((GS == GS_SHARED || GS == GS_GLOBAL) && G.direct) {  // uniform over the warp
-    if (kept) atomicAdd(GS == GS_SHARED ? &G.table[grp] : &G.gout[grp], (unsigned long long)val);
+    if (kept) {
+      if (GS == GS_SHARED) shared_add64(&G.lo[grp], &G.hi[grp], (uint64_t)val);
+      else atomicAdd(&G.gout[grp], (unsigned long long)val);
+    }
     return;
   }
   const uint32_t key = kept ? grp : 0xffffffffu;
@@ -146,7 +165,7 @@ __device__ __forceinline__ void aggregate(const GrpCtx &G, bool kept, uint32_t g
   if (!kept) return;
   const uint64_t s = peer_sum64(peers, (uint64_t)val);
   if ((threadIdx.x & 31) != (uint32_t)(__ffs(peers) - 1)) return;
-  if (GS == GS_SHARED) atomicAdd(&G.table[grp], (unsigned long long)s);
+  if (GS == GS_SHARED) shared_add64(&G.lo[grp], &G.hi[grp], s);
   else if (GS == GS_GLOBAL) atomicAdd(&G.gout[grp], (unsigned long long)s);
   else hash_add(G, grp, s);
 }
@@ -167,13 +186,14 @@ __device__ __forceinline__ GrpCtx grp_init(uint8_t *smem, uint32_t nr_grp, uint3
   G.gout = gout;
   G.hcap = hcap;
   G.direct = nr_grp >= GRP_DIRECT_MIN;
-  G.table = reinterpret_cast<unsigned long long *>(smem);
+  G.lo = reinterpret_cast<uint32_t *>(smem);
+  G.hi = G.lo + (GS == GS_HASH ? hcap : nr_grp);
   G.keys = reinterpret_cast<uint32_t *>(smem + (size_t)hcap * 8);
   if (GS == GS_SHARED)
-    for (uint32_t i = threadIdx.x; i < nr_grp; i += blockDim.x) G.table[i] = 0;
+    for (uint32_t i = threadIdx.x; i < nr_grp; i += blockDim.x) G.lo[i] = 0, G.hi[i] = 0;
   if (GS == GS_HASH)
     for (uint32_t i = threadIdx.x; i < hcap; i += blockDim.x) {
-      G.table[i] = 0;
+      G.lo[i] = 0, G.hi[i] = 0;
       G.keys[i] = HASH_EMPTY;
     }
   return G;
@@ -213,13 +233,14 @@ __device__ __forceinline__ void grp_flush(const GrpCtx &G, uint32_t nr_grp, int6
   }
   if (GS == GS_SHARED)
     for (uint32_t i = threadIdx.x; i < nr_grp; i += blockDim.x) {
-      const unsigned long long v = G.table[i];
+      const unsigned long long v = G.lo[i] | (unsigned long long)G.hi[i] << 32;
       if (v) atomicAdd(&G.gout[i], v);
     }
   if (GS == GS_HASH)
     for (uint32_t i = threadIdx.x; i < G.hcap; i += blockDim.x) {
       const uint32_t k = G.keys[i];
-      if (k != HASH_EMPTY && G.table[i]) atomicAdd(&G.gout[k], G.table[i]);
+      const unsigned long long v = G.lo[i] | (unsigned long long)G.hi[i] << 32;
+      if (k != HASH_EMPTY && v) atomicAdd(&G.gout[k], v);
     }
 }
 
