@@ -613,6 +613,19 @@ mb_status lower_query(Engine &E, const mb_query &q, const mb_plan &plan, Lowered
       L.canonical_bitmaps += d.full || d.empty ? 0 : d.nb();
     }
   }
+  // the clause of each predicate (clauses and predicates list a template's
+  // columns in their own orders; clause c's one term reads source c)
+  static const uint8_t clause_col[5][4] = {{0, 0, 0, 0},
+                                           {IC_DATE, IC_DISC, IC_QTY, IC_N},
+                                           {IC_SCITY, IC_MFGR, IC_N, IC_N},
+                                           {IC_SCITY, IC_DATE, IC_CCITY, IC_N},
+                                           {IC_SCITY, IC_DATE, IC_CCITY, IC_MFGR}};
+  for (size_t i = 0; i < L.preds.size(); ++i) {
+    const Cover &cv = L.covers[i];
+    if (cv.full || cv.empty || cv.complement || cv.chk()) continue;
+    for (uint32_t c = 0; c < L.op.nclause; ++c)
+      if (clause_col[q.tmpl][c] == L.preds[i].col) L.sure |= 1u << c;
+  }
   // predicate order: most selective first (ANDM skips loads under zero words)
   std::vector<int> order;
   for (size_t i = 0; i < L.preds.size(); ++i)
@@ -972,7 +985,7 @@ mb_status run_lowered(Engine &E, Lowered &L, const mb_plan &plan, int64_t *d_out
     MB_CHECK(mb_bitmap_to_rows(poss, chk ? unc : nullptr, E.nrows, E.rows, E.d_rowcnt, st));
     return mb_rows_grpby(E.rows, E.d_rowcnt, E.rows_cap, &L.op, L.ngroups, d_out, d_nq, st);
   }
-  return fused_grpby(&L.prg, &L.op, L.ngroups, d_out, d_nq, &plan.launch, st, zero);
+  return fused_grpby(&L.prg, &L.op, L.ngroups, d_out, d_nq, &plan.launch, st, zero, L.sure);
 }
 }  // namespace mb
 

@@ -58,6 +58,11 @@ struct Lowered {
   std::vector<Pred> preds;
   std::vector<Cover> covers;
   int col_pred[MB_MAXCOLS] = {};   // predicate (template order) of each program operand
+  // Clauses of the op (bit c) whose predicate has an exact cover of bins
+  // inside its range: every selected row satisfies them.  (A complemented or
+  // full predicate selects rows outside the index's value domain too: its
+  // clause stays checked.)
+  uint32_t sure = 0;
   uint64_t canonical_bitmaps = 0;  // plan-independent: min(direct, complement) exact cover
   // Back to the state of a fresh Lowered for the fields lowering reads before
   // writing (prg, op and mids are rewritten in full, the vectors keep their
@@ -70,6 +75,7 @@ struct Lowered {
     preds.clear();
     covers.clear();
     for (int &c : col_pred) c = 0;
+    sure = 0;
     canonical_bitmaps = 0;
   }
 };
@@ -184,9 +190,11 @@ mb_status run_lowered(Engine &E, Lowered &L, const mb_plan &plan, int64_t *d_out
 
 // p &= ~u over the words of an nrows bitmap (grpby.cu).
 mb_status certain_of(uint32_t *p, const uint32_t *u, uint64_t nrows, cudaStream_t st);
-// mb_vprg_grpby with the output zeroing optional (grpby.cu).
+// mb_vprg_grpby with the output zeroing optional (grpby.cu); sure: clauses of
+// the op (bit c) that hold for every row the program selects, so uncertain rows
+// need not be checked against them.
 mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_t *out, uint64_t *nqual,
-                      const mb_launch *launch, cudaStream_t st, bool zero);
+                      const mb_launch *launch, cudaStream_t st, bool zero, uint32_t sure = 0);
 
 }  // namespace mb
 

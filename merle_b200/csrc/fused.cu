@@ -1,4 +1,4 @@
-// fused.cu - the TMA-staged fused kernel: program -> compaction -> op ->
+// fused.cu - the fused kernels' evaluators of any op, and the TMA-staged kernel: program -> compaction -> op ->
 // group-by, with every operand bitmap of a tile staged in shared memory.
 //
 // Reference: vprg_grpby (primitive.cuh:340-445).  The reference reads each
@@ -28,6 +28,7 @@
 #include "opeval.cuh"
 #include "tma.cuh"
 #include "vbp.cuh"
+#include "fused_warp.cuh"
 
 namespace mb {
 
@@ -83,22 +84,26 @@ __device__ __forceinline__ void load_row(const mb_op &O, uint32_t need, uint32_t
   }
 }
 
+// The op's filter over loaded values.
+__device__ __forceinline__ bool filter_row(const mb_op &O, const uint32_t (&v)[MB_MAXSRC], uint32_t bad) {
+  uint32_t t = 0;
+  for (uint32_t c = 0; c < O.nclause; ++c) {
+    bool any = false;
+    const uint32_t len = O.clause_len[c];
+    for (uint32_t k = 0; k < len; ++k, ++t) {
+      const mb_term &tm = O.terms[t];
+      const uint64_t x = pick(v, tm.src);
+      any |= !((bad >> tm.src) & 1u) && x >= tm.lo && x < tm.hi;
+    }
+    if (!any) return false;
+  }
+  return true;
+}
+
 // The op over loaded values (the same semantics as op_eval in opeval.cuh).
 __device__ __forceinline__ bool eval_row(const mb_op &O, const uint32_t (&v)[MB_MAXSRC], uint32_t bad, bool chk,
                                          uint32_t nr_grp, int64_t &value, uint32_t &group) {
-  if (chk) {
-    uint32_t t = 0;
-    for (uint32_t c = 0; c < O.nclause; ++c) {
-      bool any = false;
-      const uint32_t len = O.clause_len[c];
-      for (uint32_t k = 0; k < len; ++k, ++t) {
-        const mb_term &tm = O.terms[t];
-        const uint64_t x = pick(v, tm.src);
-        any |= !((bad >> tm.src) & 1u) && x >= tm.lo && x < tm.hi;
-      }
-      if (!any) return false;
-    }
-  }
+  if (chk && !filter_row(O, v, bad)) return false;
   uint32_t g = 0;
   for (uint32_t k = 0; k < O.nkey; ++k) {
     const mb_key &kk = O.keys[k];
@@ -310,85 +315,26 @@ __device__ __forceinline__ void compact_chunk(const mb_op &O, const OpNeeds &N, 
   __syncwarp();
 }
 
-// The conjunctive chain on words w0 + k*32 + lane (k < V): every bitmap of the
-// chain is loaded in batches of 8 independent coalesced loads, so a warp tile
-// costs one memory round trip per 8 bitmaps (the interpreter's ANDM chain
-// costs one per operand).
-template <int V, bool CHK>
-__device__ __forceinline__ void cnf_words(const DevPrg &P, uint64_t w0, uint32_t (&p)[V], uint32_t (&u)[V]) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint32_t acc[V], cur[V], ce[V], unc[V];
-#pragma unroll
-  for (int k = 0; k < V; ++k) acc[k] = 0xffffffffu, cur[k] = ce[k] = unc[k] = 0;
-  const uint32_t nb = P.ncnf;
-  for (uint32_t b0 = 0; b0 < nb; b0 += 8) {
-    uint32_t x[8][V];
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int k = 0; k < V; ++k) {
-        const uint64_t w = w0 + k * 32 + lane;
-        x[j][k] = (b0 + j < nb && w < P.nwords) ? __ldcs(P.cnf_ptr[b0 + j] + w) : 0u;
-      }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (b0 + j >= nb) break;
-      const uint32_t f = P.cnf_flag[b0 + j];
-#pragma unroll
-      for (int k = 0; k < V; ++k) {
-        cur[k] |= x[j][k];
-        if (f & CNF_EDGE) ce[k] |= x[j][k];
-      }
-      if (f & CNF_END) {
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-          acc[k] &= (f & CNF_NEG) ? ~cur[k] : cur[k];
-          if (CHK && !(f & CNF_NEG)) unc[k] |= ce[k];
-          cur[k] = ce[k] = 0;
-        }
-      }
-    }
+// Any op as the warp-independent kernel's drain (fused_warp.cuh).
+template <bool CHK, int GS>
+struct AnyDrain {
+  const mb_op &O;
+  OpNeeds N;
+  uint32_t nr_grp;
+  __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, bool, const GrpCtx &G, int64_t &acc,
+                                        uint32_t &cnt) const {
+    uint64_t c = 0;
+    drain64<CHK, GS>(O, N, q, n, nr_grp, G, acc, c);
+    cnt += (uint32_t)c;
   }
-  const uint32_t tail = (uint32_t)(P.nrows & 31u);
-#pragma unroll
-  for (int k = 0; k < V; ++k) {
-    const uint64_t w = w0 + k * 32 + lane;
-    uint32_t m = w < P.nwords ? 0xffffffffu : 0u;
-    if (tail && w + 1 == P.nwords) m = (1u << tail) - 1u;
-    p[k] = acc[k] & m;
-    u[k] = CHK ? (unc[k] & p[k]) : 0u;
-  }
-}
+};
 
-// Warp-independent fused kernel for conjunctive programs: each warp walks
-// tiles of 32*V words on its own (no block barrier until the final flush):
-// load the chain's words, compact 32-word chunks into its queue, drain.
 template <int V, bool CHK, int GS>
-__global__ void __launch_bounds__(FT_THREADS)
+__global__ void __launch_bounds__(FW_THREADS)
 fused_warp_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ mb_op O, OpNeeds N, uint32_t nr_grp,
                   uint32_t hcap, unsigned long long *__restrict__ out, unsigned long long *__restrict__ nqual) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ uint64_t red[64];
-  const uint32_t warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const size_t gbytes = (grp_smem_bytes(GS, nr_grp, hcap) + 15) & ~(size_t)15;
-  GrpCtx G = grp_init<GS>(smem, nr_grp, hcap, out);
-  uint32_t *queue = reinterpret_cast<uint32_t *>(smem + gbytes) + (size_t)warp * FT_QCAP;
-  __syncthreads();
-  int64_t acc = 0;
-  uint64_t cnt = 0;
-  uint32_t qn = 0;
-  constexpr uint32_t TW = 32 * V;
-  const uint64_t ntiles = (P.nwords + TW - 1) / TW;
-  for (uint64_t t = (uint64_t)blockIdx.x * nw + warp; t < ntiles; t += (uint64_t)gridDim.x * nw) {
-    uint32_t p[V], u[V];
-    cnf_words<V, CHK>(P, t * TW, p, u);
-#pragma unroll
-    for (int k = 0; k < V; ++k)
-      compact_chunk<CHK, GS>(O, N, queue, qn, t * TW + k * 32, p[k], u[k], nr_grp, G, acc, cnt);
-  }
-  if (qn) drain64<CHK, GS>(O, N, queue, qn, nr_grp, G, acc, cnt);
-  __syncthreads();
-  grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
+  extern __shared__ __align__(128) uint8_t smem[];
+  fused_warp_body<V, CHK, GS>(P, AnyDrain<CHK, GS>{O, N, nr_grp}, nr_grp, hcap, out, nqual, smem);
 }
 
 // T = FT_THREADS * V words per CTA tile.
@@ -573,24 +519,9 @@ bool fused_warp_applies(const DevPrg &P, const mb_op &O) {
 template <int V, bool CHK, int GS>
 static mb_status launch_fw(const DevPrg &P, const mb_op &O, uint32_t nr_grp, uint32_t hcap, int64_t *out,
                            uint64_t *nq, uint32_t warps, uint32_t cps, cudaStream_t st) {
-  auto kern = fused_warp_kernel<V, CHK, GS>;
-  const size_t smem = ((grp_smem_bytes(GS, nr_grp, hcap) + 15) & ~(size_t)15) + (size_t)warps * FT_QCAP * 4;
-  const DevInfo &di = dev_info();
-  if (smem > (size_t)di.max_smem_optin) return fail(MB_ERR_INVALID, "fused: %zu bytes of shared memory", smem);
-  MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int occ = 0;
-  MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, (int)(warps * 32), smem));
-  if (occ < 1) return fail(MB_ERR_INVALID, "fused: kernel does not fit on an SM");
-  if (cps && (int)cps < occ) occ = (int)cps;
-  const uint64_t ntiles = (P.nwords + 32 * V - 1) / (32 * V);
-  uint64_t grid = (uint64_t)di.sms * occ;
-  const uint64_t need = (ntiles + warps - 1) / warps;
-  if (grid > need) grid = need ? need : 1;
-  kern<<<(unsigned)grid, warps * 32, smem, st>>>(P, O, op_needs(O), nr_grp, hcap,
-                                                 reinterpret_cast<unsigned long long *>(out),
-                                                 reinterpret_cast<unsigned long long *>(nq));
-  MB_LAUNCH_CHECK("fused_warp_kernel");
-  return MB_OK;
+  return fw_launch(fused_warp_kernel<V, CHK, GS>, V, P.nwords, grp_smem_bytes(GS, nr_grp, hcap), warps, cps, st,
+                   P, O, op_needs(O), nr_grp, hcap, reinterpret_cast<unsigned long long *>(out),
+                   reinterpret_cast<unsigned long long *>(nq));
 }
 
 template <int V, bool CHK>
@@ -604,11 +535,73 @@ static mb_status fw_gs(int gs, const DevPrg &P, const mb_op &O, uint32_t nr_grp,
   }
 }
 
-mb_status fused_warp(const DevPrg &P, const mb_op &O, uint32_t nr_grp, int gs, uint32_t hcap, uint32_t V,
-                     uint32_t warps, int64_t *out, uint64_t *nq, uint32_t cps, cudaStream_t st) {
-  if (V == 0) V = 2;
-  if (warps == 0 || warps > 8) warps = 8;  // FT_THREADS bounds the block
+int shape_of(const mb_op &O, uint32_t nr_grp, uint32_t sure, ShapeArgs *A, bool *narrow) {
+  memset(A, 0, sizeof(*A));
+  A->ng = nr_grp;
+  if (O.nsrc > 6) return -1;
+  const OpNeeds N = op_needs(O);
+  uint32_t keym = 0, yearm = 0, termm = 0;
+  for (uint32_t c = 0; c < O.nclause; ++c) {
+    if (O.clause_len[c] != 1) return -1;
+    const mb_term &t = O.terms[c];
+    if ((termm >> t.src) & 1u || t.lo >= t.hi || t.lo > 0xffffffffull) return -1;
+    termm |= 1u << t.src;
+    if (!((sure >> c) & 1u)) A->fmask |= 1u << t.src;
+    A->lo[t.src] = (uint32_t)t.lo;
+    A->hi[t.src] = t.hi > 0x100000000ull ? 0xffffffffu : (uint32_t)(t.hi - 1);
+  }
+  for (uint32_t k = 0; k < O.nkey; ++k) {
+    const mb_key &kk = O.keys[k];
+    if (kk.src > 3 || (keym >> kk.src) & 1u) return -1;
+    keym |= 1u << kk.src;
+    ShapeKey &K = A->key[kk.src];
+    if (kk.xform == MB_X_YEAR) yearm |= 1u << kk.src;
+    const uint32_t d = kk.xform == MB_X_DIV ? kk.div : 1u;
+    if (d == 0) return -1;
+    const DivMagic m = div_magic(d);
+    K = ShapeKey{m.m, m.sh1, m.sh2, kk.base, kk.mul, d == 1 ? 1u : 0u};
+  }
+  for (uint32_t i = 0; i < BNSHAPE; ++i) {
+    const BShape &b = BSHAPES[i];
+    if (b.ns != O.nsrc || b.kv != N.kv_mask || b.filt != N.filt_mask || b.filt != termm || b.keym != keym ||
+        b.yearm != yearm || b.vk != O.vkind || b.va != O.va || (b.vk != MB_V_COL && b.vb != O.vb))
+      continue;
+    for (int nar = 0; nar < 2; ++nar) {
+      bool same = true;
+      for (uint32_t s = 0; s < b.ns && same; ++s) same = !O.src[s].fk && O.src[s].width == SHAPE_W[i][nar][s];
+      if (!same) continue;
+      for (uint32_t s = 0; s < b.ns; ++s) A->col[s] = O.src[s].col;
+      *narrow = nar != 0;
+      return (int)i;
+    }
+  }
+  return -1;
+}
+
+mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, uint32_t nr_grp, int gs, uint32_t hcap,
+                     uint32_t V, uint32_t warps, int64_t *out, uint64_t *nq, uint32_t cps, cudaStream_t st) {
+  // Words a lane: wider tiles mean fewer, wider loads and fewer warps at work.
+  // Device time at V = 1 / 2 / 4: 13 SSB queries, 1M rows 179 / 185 / 189 us,
+  // 120M rows 997 / 879 / 871 us; a 24-query spanning mix, 60M rows 1,735 /
+  // 1,496 / 1,555 us; the 64-query spanning mix, 600M rows - / 43.8 / 41.1 ms.
+  if (V == 0) V = P.nrows < 4000000 ? 1 : P.nrows < 200000000 ? 2 : 4;
+  if (warps == 0 || warps > 8) warps = 8;  // FW_THREADS bounds the block
+  if (!vec4) V = 1;                        // unaligned bitmaps: word loads
   const bool chk = P.chk != 0;
+  ShapeArgs A;
+  bool narrow = false;
+  const int sh = gs == GS_HASH ? -1 : shape_of(O, nr_grp, sure, &A, &narrow);
+  // a compiled op: one group in a register (shape 1), or several in a table
+  if (sh >= 0 && (sh == 0 ? gs == GS_SCALAR : gs != GS_SCALAR && nr_grp >= GRP_DIRECT_MIN)) {
+    const ShapeLaunch L{nr_grp, V, warps, cps, gs, narrow, reinterpret_cast<unsigned long long *>(out),
+                        reinterpret_cast<unsigned long long *>(nq), st};
+    switch (sh) {
+    case 0: return fused_shape1(P, A, L);
+    case 1: return fused_shape2(P, A, L);
+    case 2: return fused_shape3(P, A, L);
+    default: return fused_shape4(P, A, L);
+    }
+  }
   if (V == 4) return chk ? fw_gs<4, true>(gs, P, O, nr_grp, hcap, out, nq, warps, cps, st)
                          : fw_gs<4, false>(gs, P, O, nr_grp, hcap, out, nq, warps, cps, st);
   if (V == 2) return chk ? fw_gs<2, true>(gs, P, O, nr_grp, hcap, out, nq, warps, cps, st)

@@ -1,0 +1,9 @@
+// fused_shape2.cu - the fused kernels of op shape 2 (query template 2): see
+// fused_warp.cuh and shape.cuh.  One file per shape, so that they compile side by side.
+#include "fused_warp.cuh"
+
+namespace mb {
+mb_status fused_shape2(const DevPrg &P, const ShapeArgs &A, const ShapeLaunch &L) {
+  return fused_shape_launch<1>(P, A, L);
+}
+}  // namespace mb

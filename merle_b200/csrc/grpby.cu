@@ -598,7 +598,7 @@ using namespace mb;
 
 namespace mb {
 mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_t *out, uint64_t *nqual,
-                      const mb_launch *launch, cudaStream_t st, bool zero) {
+                      const mb_launch *launch, cudaStream_t st, bool zero, uint32_t sure) {
   if (!out || !nqual) return fail(MB_ERR_INVALID, "mb_vprg_grpby: NULL output");
   if (nr_grp == 0) return fail(MB_ERR_INVALID, "mb_vprg_grpby: nr_grp == 0");
   const int chk = !mb_vprg_is_nochk(p);
@@ -620,7 +620,7 @@ mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_
     return fail(MB_ERR_INVALID, "mb_vprg_grpby: words_per_lane %u", L.words_per_lane);
   const uint32_t hcap = DEFAULT_HCAP;
   if (L.staging == MB_STAGE_AUTO && fused_warp_applies(P, *op))
-    return fused_warp(P, *op, nr_grp, gs, hcap, L.words_per_lane, L.warps_per_cta, out, nqual, L.ctas_per_sm, st);
+    return fused_warp(P, v4, *op, sure, nr_grp, gs, hcap, L.words_per_lane, L.warps_per_cta, out, nqual, L.ctas_per_sm, st);
   if (L.staging == MB_STAGE_TMA && fused_tma_applies(P, v4, *op)) {
     const mb_status r = fused_tma(P, *op, nr_grp, gs, hcap, L.words_per_lane, out, nqual, L.ctas_per_sm, st);
     if (r != MB_ERR_UNSUPPORTED) return r;  // else: too many bitmaps to stage, load directly
@@ -638,7 +638,7 @@ mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_
 
 extern "C" mb_status mb_vprg_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_t *out,
                                    uint64_t *nqual, const mb_launch *launch, void *stream) {
-  return fused_grpby(p, op, nr_grp, out, nqual, launch, as_stream(stream), true);
+  return fused_grpby(p, op, nr_grp, out, nqual, launch, as_stream(stream), true, 0);
 }
 
 // The clause that screens rows in the no-index scan: the first whose terms

@@ -221,6 +221,7 @@ struct OpNeeds {
   uint32_t kv_mask, filt_mask;
 };
 OpNeeds op_needs(const mb_op &O);
-mb_status fused_warp(const DevPrg &P, const mb_op &O, uint32_t nr_grp, int gs, uint32_t hcap, uint32_t V,
-                     uint32_t warps, int64_t *out, uint64_t *nq, uint32_t cps, cudaStream_t st);
+// sure: clauses of the op (bit c) that hold for every row the program selects.
+mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, uint32_t nr_grp, int gs, uint32_t hcap,
+                     uint32_t V, uint32_t warps, int64_t *out, uint64_t *nq, uint32_t cps, cudaStream_t st);
 }  // namespace mb
