@@ -175,8 +175,10 @@ def _run_timed(eng, qs, plans, out, nq) -> np.ndarray:
 
 
 def measure_candidates(eng, qs, reps: int = 3, chunk: int = 512, cands=range(NC)) -> np.ndarray:
-    """times[i, c] = median over reps of query i's device time (ms) under
-    candidate c.  Candidates that lower to the same plan as an earlier one are
+    """times[i, c] = the least over reps of query i's device time (ms) under
+    candidate c (what disturbs a timing only adds to it: at 24M rows a network
+    trained on the least of three gains 1.010-1.018x over the rule plan, on
+    the median 1.007-1.012x).  Candidates that lower to the same plan as an earlier one are
     timed once and share its figure (so identical plans never look different
     through timing noise)."""
     from . import device as D
@@ -202,10 +204,10 @@ def measure_candidates(eng, qs, reps: int = 3, chunk: int = 512, cands=range(NC)
                 part = idx[s:s + chunk]
                 t = _run_timed(eng, [qs[i] for i in part], [plans[i][j] for i in part], out, nq)
                 samples[r, part, j] = t
-    med = np.median(samples, axis=0)
+    least = samples.min(axis=0)
     for i in range(n):
-        med[i] = med[i, rep_of[i]]
-    return med
+        least[i] = least[i, rep_of[i]]
+    return least
 
 
 def targets(times: np.ndarray) -> tuple[np.ndarray, np.ndarray]:
