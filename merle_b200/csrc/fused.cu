@@ -329,12 +329,12 @@ struct AnyDrain {
   }
 };
 
-template <int V, bool CHK, int GS>
+template <int V, bool CHK, int GS, bool CNF>
 __global__ void __launch_bounds__(FW_THREADS)
 fused_warp_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ mb_op O, OpNeeds N, uint32_t nr_grp,
                   uint32_t hcap, unsigned long long *__restrict__ out, unsigned long long *__restrict__ nqual) {
   extern __shared__ __align__(128) uint8_t smem[];
-  fused_warp_body<V, CHK, GS>(P, AnyDrain<CHK, GS>{O, N, nr_grp}, nr_grp, hcap, out, nqual, smem);
+  fused_warp_body<V, CHK, GS, CNF>(P, AnyDrain<CHK, GS>{O, N, nr_grp}, nr_grp, hcap, out, nqual, smem);
 }
 
 // T = FT_THREADS * V words per CTA tile.
@@ -510,7 +510,7 @@ mb_status fused_tma(const DevPrg &P, const mb_op &O, uint32_t nr_grp, int gs, ui
 
 // ------------------------------------------------- warp-independent kernel
 bool fused_warp_applies(const DevPrg &P, const mb_op &O) {
-  if (!P.cnf || P.nrows == 0) return false;
+  if (P.nrows == 0 || P.nrows >= (1ull << 31)) return false;  // (bit 31 of a queued row: uncertain)
   for (uint32_t s = 0; s < O.nsrc; ++s)
     if (O.src[s].width > 4) return false;
   return true;
@@ -519,9 +519,11 @@ bool fused_warp_applies(const DevPrg &P, const mb_op &O) {
 template <int V, bool CHK, int GS>
 static mb_status launch_fw(const DevPrg &P, const mb_op &O, uint32_t nr_grp, uint32_t hcap, int64_t *out,
                            uint64_t *nq, uint32_t warps, uint32_t cps, cudaStream_t st) {
-  return fw_launch(fused_warp_kernel<V, CHK, GS>, V, P.nwords, grp_smem_bytes(GS, nr_grp, hcap), warps, cps, st,
-                   P, O, op_needs(O), nr_grp, hcap, reinterpret_cast<unsigned long long *>(out),
-                   reinterpret_cast<unsigned long long *>(nq));
+  auto go = [&](auto kern) {
+    return fw_launch(kern, V, P.nwords, grp_smem_bytes(GS, nr_grp, hcap), warps, cps, st, P, O, op_needs(O), nr_grp,
+                     hcap, reinterpret_cast<unsigned long long *>(out), reinterpret_cast<unsigned long long *>(nq));
+  };
+  return P.cnf ? go(fused_warp_kernel<V, CHK, GS, true>) : go(fused_warp_kernel<V, CHK, GS, false>);
 }
 
 template <int V, bool CHK>
@@ -590,7 +592,7 @@ mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, 
   const bool chk = P.chk != 0;
   ShapeArgs A;
   bool narrow = false;
-  const int sh = gs == GS_HASH ? -1 : shape_of(O, nr_grp, sure, &A, &narrow);
+  const int sh = gs == GS_HASH || !P.cnf ? -1 : shape_of(O, nr_grp, sure, &A, &narrow);
   // a compiled op: one group in a register (shape 1), or several in a table
   if (sh >= 0 && (sh == 0 ? gs == GS_SCALAR : gs != GS_SCALAR && nr_grp >= GRP_DIRECT_MIN)) {
     const ShapeLaunch L{nr_grp, V, warps, cps, gs, narrow, reinterpret_cast<unsigned long long *>(out),

@@ -1,4 +1,4 @@
-// fused_warp.cuh - the warp-independent fused kernel for conjunctive programs
+// fused_warp.cuh - the warp-independent fused kernel
 // (program -> compaction -> op -> group-by), over the drains of fused.cu (any
 // op) and shape.cuh (compiled ops).
 //
@@ -143,7 +143,11 @@ __device__ __forceinline__ void fw_compact(const DR &dr, uint32_t *queue, uint32
   __syncwarp();
 }
 
-template <int V, bool CHK, int GS, class DR>
+// CNF: the program is a conjunctive chain (fw_chain); else its instructions run
+// one by one (vbp_eval) on the lane's words.  (A program with an OR and checked
+// edges over 60M rows, 256 groups: 236 us in the kernel whose drain walks the op
+// source by source, 163 us here with each row's loads issued together.)
+template <int V, bool CHK, int GS, bool CNF, class DR>
 __device__ __forceinline__ void fused_warp_body(const DevPrg &P, const DR &dr, uint32_t nr_grp, uint32_t hcap,
                                                 unsigned long long *out, unsigned long long *nqual, uint8_t *smem) {
   __shared__ uint64_t red[64];
@@ -158,7 +162,8 @@ __device__ __forceinline__ void fused_warp_body(const DevPrg &P, const DR &dr, u
   const uint64_t ntiles = (P.nwords + TW - 1) / TW;
   for (uint64_t t = (uint64_t)blockIdx.x * nw + warp; t < ntiles; t += (uint64_t)gridDim.x * nw) {
     uint32_t p[V], u[V];
-    fw_chain<V, CHK>(P, t * TW, p, u);
+    if (CNF) fw_chain<V, CHK>(P, t * TW, p, u);
+    else vbp_eval<V, CHK>(P, t * TW + lane * V, p, u);
     const uint32_t rb = (uint32_t)((t * TW + lane * V) * 32);
 #pragma unroll
     for (int k = 0; k < V; ++k)
@@ -185,7 +190,7 @@ __global__ void __launch_bounds__(FW_THREADS, 3)
 fused_shape_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ ShapeArgs A, uint32_t nr_grp,
                    unsigned long long *__restrict__ out, unsigned long long *__restrict__ nqual) {
   extern __shared__ __align__(128) uint8_t smem[];
-  fused_warp_body<V, CHK, GS>(P, ShapeDrain<SH, NARROW, CHK, GS>{A}, nr_grp, 0, out, nqual, smem);
+  fused_warp_body<V, CHK, GS, true>(P, ShapeDrain<SH, NARROW, CHK, GS>{A}, nr_grp, 0, out, nqual, smem);
 }
 
 // Launch of a warp-independent kernel of `warps` warps: persistent grid.

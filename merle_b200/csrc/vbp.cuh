@@ -38,7 +38,8 @@ struct DevPrg {
 enum { CNF_EDGE = 1, CNF_END = 2, CNF_NEG = 4 };
 
 // Host: validates and flattens an mb_vprg.  vec4 = every bitmap pointer is
-// 16-byte aligned (128-bit loads allowed).
+// 16-byte aligned (64- and 128-bit loads of words at multiples of 2 and 4
+// allowed).
 mb_status flatten_prg(const mb_vprg *p, int chk, DevPrg *out, bool *vec4);
 // Host: sets cnf / cmask / neg when the program is a conjunctive chain.
 void detect_cnf(DevPrg *o);
@@ -48,6 +49,9 @@ __device__ __forceinline__ void vload(const uint32_t *p, uint64_t w0, uint64_t n
   if (V == 4 && w0 + 4 <= nwords) {
     uint4 t = ld_stream4(p + w0);
     o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
+  } else if (V == 2 && w0 + 2 <= nwords) {
+    const uint2 t = __ldcs(reinterpret_cast<const uint2 *>(p + w0));
+    o[0] = t.x; o[1] = t.y;
   } else {
 #pragma unroll
     for (int k = 0; k < V; ++k) o[k] = (w0 + k < nwords) ? __ldcs(p + w0 + k) : 0u;
@@ -213,7 +217,8 @@ mb_status fused_tma(const DevPrg &P, const mb_op &O, uint32_t nr_grp, int gs, ui
 }  // namespace mb
 
 namespace mb {
-// The warp-independent kernel for conjunctive programs (fused.cu).
+// The warp-independent kernel (fused.cu): any program over an op whose sources
+// have at most 4 bytes.
 bool fused_warp_applies(const DevPrg &P, const mb_op &O);
 // Which op sources every row needs (keys, value) and which only uncertain
 // rows need (filter terms).

@@ -87,3 +87,47 @@ def test_covers_agree(oracle_answers, cuda, cover):
             assert gn == wn
     finally:
         e.close()
+
+
+PROGRAMS = {  # general programs (not a conjunctive chain), with and without edge bins
+    "or_and": ([abi.ORM, 0, 0, 0], [abi.ORM, 0, 1, 0], [abi.ANDM, 0, 2, 0]),
+    "not_or": ([abi.ORM, 1, 0, 0], [abi.NOT, 0, 1, 0], [abi.ORM, 0, 1, 0]),
+    "regs": ([abi.ORM, 0, 0, 0], [abi.ORM, 1, 1, 0], [abi.ORM, 2, 2, 0], [abi.AND, 0, 1, 0], [abi.OR, 0, 2, 0]),
+}
+
+
+@pytest.mark.parametrize("chk", [False, True])
+@pytest.mark.parametrize("n", [1, 1023, 2049, 40_003])
+def test_general_programs_match_oracle(orc, cuda, n, chk):
+    """Programs outside the conjunctive form in the warp-independent kernel, at
+    every tile width and group strategy, against the oracle's interpreter."""
+    from merle_b200 import device as D, ops
+    f, fd = orc.gen_flat(11, n), D.DevFlat(11, n)
+    s = abi.mb_src()
+    bm_h, bm_d = [], []
+    for col, lo, hi in (("a", [0, 300, 600], [300, 600, 700]), ("b", [0, 2, 9], [2, 9, 30]), ("c", [1, 20, 30], [20, 30, 51])):
+        s.col, s.width = orc.ptr(f[col]), 4
+        h, _ = orc.bitmap_create(s, n, lo, hi)
+        d, _ = D.bitmap_create(D.src_of(fd[col]), n, lo, hi)
+        bm_h.append(h)
+        bm_d.append(d)
+    args = (200, 650, list(range(1, 20)), 0, 40)  # a filter, an OR clause, group-less SUM
+
+    def prog(b, ins):
+        return ops.Vprg(n, [ops.Col(middle=[x[0], x[1]], rightmost=x[2] if chk else None) for x in b],
+                        [tuple(i) for i in ins]).to_c()
+
+    def op(c):
+        o = ops.flat_op(c["a"], c["b"], c["c"], c["d"], c["e"], args[0], args[1], [3, 7, 11], args[3], args[4])
+        o.keys = [(3, abi.X_ID, 1, 0, 1)]
+        return o.to_c()
+    for name, ins in PROGRAMS.items():
+        want, wn = orc.vprg_grpby(prog(bm_h, ins), op(f), 11)
+        pd, od = prog(bm_d, ins), op(fd)
+        for v in (0, 1, 2, 4):
+            for gs in (abi.GRP_AUTO, abi.GRP_GLOBAL, abi.GRP_HASH):
+                la = abi.mb_launch()
+                la.words_per_lane, la.grp_strategy = v, gs
+                out, nq = D.vprg_grpby(pd, od, 11, la)
+                np.testing.assert_array_equal(D.to_host(out, np.int64), want, err_msg=f"{name} V={v} gs={gs}")
+                assert int(D.to_host(nq, np.uint64)[0]) == wn
