@@ -11,20 +11,28 @@
 // of equal all-0 / all-1 groups is one fill (wahCmprsCPU's output).
 //
 // The reference builds its GPU side from moderngpu passes (transform_scan,
-// transform_lbs, transform_compact; merle/wahGpuCmprs.cu).  Here:
-//   encode  (1) per-block count of stream words (a group starts a word when
-//           it is a literal or differs in kind from the group before it);
-//           (2) one CTA scans the block counts; (3) each block writes its
-//           words, each with its starting group in a side array; (4) a
-//           fill's run = the next word's starting group minus its own.
-//   decode  (1)-(2) the exclusive scan of the words' group counts (what
-//           wahCntExcScan computes, merle/wahGpuCmprs.cu:6-14); (3) for each
-//           block of output words, the stream words covering its groups by
-//           binary search over that scan; (4) each output word w holds rows
-//           32w .. 32w+31 = the tail of group floor(32w/31) and the head of
-//           the next one: the block stages its stream words in shared memory
-//           and each thread finds its two groups there.
-// All passes are HBM-bound integer work: no tensor cores.
+// transform_lbs, transform_compact; merle/wahGpuCmprs.cu).  Here every pass works
+// on blocks of 4,096 groups = 3,968 bitmap words, so that groups and words meet at
+// block boundaries, and a thread on 32 groups = 31 words, so that every shift
+// between the two is a constant:
+//   encode  (1) per block the stream words its groups start (a group starts a
+//           word when it is a literal or differs in kind from the group before
+//           it): three 32-bit masks a thread; (2) each block writes its words,
+//           fills with the run they have inside the block, through a
+//           shared-memory buffer; (3) a block whose first groups continue the
+//           run before it adds them to that fill.
+//   decode  (1) group counts per block of stream words; (2) each word's first
+//           group (what wahCntExcScan computes, merle/wahGpuCmprs.cu:6-14): the
+//           word under every 4,096th group is noted; (3) each block of groups
+//           expands the words between two notes in shared memory and composes
+//           its bitmap words.
+//   AND / OR / XOR: (1)-(2) of both streams, then the encoder on the groups
+//           expanded from them; no bitmap is written.
+// What bounds the passes is instruction issue and, at 6 to 40 microseconds each,
+// the latency of a block's steps and the launches.
+// 120M rows, three predicate bitmaps compressed, ANDed and the result expanded:
+// 690 us with a thread per group and a binary search per output block, 373 us;
+// two 600M-row bitmaps of 1 % non-zero words: 702 -> 324 us.
 #include <string.h>
 #include <stdio.h>
 #include <vector>
@@ -33,44 +41,37 @@
 namespace mb {
 namespace {
 
-constexpr uint32_t WT = 256;          // threads of the counting / writing passes
-constexpr uint32_t WI = 8;            // groups (encode) or stream words (decode) per thread
+constexpr uint32_t WT = 256;          // threads of the stream-counting and direct passes
+constexpr uint32_t WI = 16;           // stream words per thread there
 constexpr uint32_t WB = WT * WI;      // per block
-constexpr uint32_t EW = WB * 31 / 32;  // bitmap words an encode block covers (2048 groups = 1984 words)
-constexpr uint32_t DT = 256;          // threads of a decode block
-constexpr uint32_t DV = 8;            // output words a decode thread writes
-constexpr uint32_t DW = DT * DV;      // output words a decode block writes
-constexpr uint32_t DCAP = 2304;       // stream words a decode block stages
-constexpr uint32_t DGRP = DW * 32 / 31 + 3;  // groups a decode block's words span
-constexpr uint32_t DLONG = 64;        // runs longer than 32 groups a decode block fills together
+constexpr uint32_t GT = 128;          // threads of a group block
+constexpr uint32_t GB = 32 * GT;      // its groups
+constexpr uint32_t GW = 31 * GT;      // its bitmap words
+constexpr uint32_t GLONG = 64;        // runs longer than 32 groups a group block fills together
 constexpr uint32_t FILL = 0x80000000u, ONES = 0x40000000u, CNT = 0x3fffffffu, LIT = 0x7fffffffu;
 constexpr uint64_t MAX_GROUPS = CNT;  // a run must fit the 30-bit count
 constexpr uint32_t WAH_MAGIC = 0x44f8a1efu;
-
-// Groups of one bitmap, or of op(a, b) over two (0 AND, 1 OR, 2 XOR).
-struct EncSrc {
-  const uint32_t *a, *b;
-  uint32_t op, order;
-  uint64_t nrows, nw;  // rows; words of a (and b): ceil(nrows / 32)
-};
-
-__device__ __forceinline__ uint32_t enc_word(const EncSrc &S, uint64_t i) {
-  if (i >= S.nw) return 0u;
-  uint32_t v = __ldg(S.a + i);
-  if (S.b) {
-    const uint32_t u = __ldg(S.b + i);
-    v = S.op == 0 ? v & u : S.op == 1 ? v | u : v ^ u;
-  }
-  return v;
-}
+// Blocks up to which a pass sums the block counts before its own itself instead
+// of after a scan launch (at most 64 KB of counts read by each).
+constexpr uint64_t DIRECT_SUM = 8192;
+// mb_wah_op's automatic choice: groups per stream word from which the direct form
+// is taken.  19.4M groups, both streams' words against the time of the explicit /
+// direct form: 747K 139 / 250 us, 76K 138 / 165, 7.6K 152 / 144, 746 164 / 90; at
+// 645K groups and fewer the explicit form is never behind.
+constexpr uint64_t DIRECT_RATIO = 2048;
 
 __device__ __forceinline__ uint32_t kind_of(uint32_t v) { return v == 0 ? 0u : v == LIT ? 1u : 2u; }
+__device__ __forceinline__ uint64_t word_groups(uint32_t w) { return (w & FILL) ? (w & CNT) : 1u; }
+__device__ __forceinline__ uint32_t group_value(uint32_t word, uint32_t order) {
+  uint32_t x = (word & FILL) ? ((word & ONES) ? LIT : 0u) : (word & LIT);
+  return order ? __brev(x) >> 1 : x;
+}
 
-// Block-wide exclusive scan of one value per thread; returns the thread's
-// prefix and sets *total.  All WT threads call it.
-template <typename T>
+// Block-wide exclusive scan of one value per thread of N threads; returns the
+// thread's prefix and sets *total.
+template <uint32_t N, typename T>
 __device__ __forceinline__ T block_excl_scan(T x, T *total) {
-  __shared__ T warp_sum[WT / 32];
+  __shared__ T warp_sum[N / 32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T inc = x;
 #pragma unroll
@@ -82,64 +83,13 @@ __device__ __forceinline__ T block_excl_scan(T x, T *total) {
   __syncthreads();
   T before = 0, all = 0;
 #pragma unroll
-  for (uint32_t i = 0; i < WT / 32; ++i) {
+  for (uint32_t i = 0; i < N / 32; ++i) {
     if (i < warp) before += warp_sum[i];
     all += warp_sum[i];
   }
   __syncthreads();  // warp_sum is reused by the next call
   *total = all;
   return before + inc - x;
-}
-
-// Stages the bitmap words of encode block b (groups [WB b, WB (b + 1)) are
-// rows [63488 b, 63488 (b + 1)) = words [EW b, EW (b + 1))) in shared memory:
-// st[0] = word EW b - 1 (the group before the block ends in it), st[1 + i] =
-// word EW b + i, st[EW + 1] = the word after.  Rows >= nrows read as 0.
-__device__ __forceinline__ void enc_stage(const EncSrc &S, uint64_t b, uint32_t *st) {
-  constexpr uint32_t R = (EW + 2 + WT - 1) / WT;
-  const int64_t base = (int64_t)(b * EW) - 1;
-  uint32_t v[R];
-#pragma unroll
-  for (uint32_t r = 0; r < R; ++r) {  // every load issued before the first store
-    const uint32_t i = r * WT + threadIdx.x;
-    const int64_t w = base + i;
-    v[r] = i < EW + 2 && w >= 0 && (uint64_t)w < S.nw ? enc_word(S, (uint64_t)w) : 0u;
-  }
-#pragma unroll
-  for (uint32_t r = 0; r < R; ++r) {
-    const uint32_t i = r * WT + threadIdx.x;
-    if (i >= EW + 2) break;
-    const int64_t w = base + i;
-    const uint64_t r0 = (uint64_t)w * 32;
-    if (w >= 0 && (uint64_t)w < S.nw && r0 + 32 > S.nrows) v[r] &= (1u << (S.nrows - r0)) - 1u;
-    st[i] = v[r];
-  }
-  __syncthreads();
-}
-
-// Local group j (-1 = the group before the block) from the staged words.
-__device__ __forceinline__ uint32_t enc_group(const uint32_t *st, int32_t j, uint32_t order) {
-  const uint32_t bit = (uint32_t)(32 + 31 * j), w = bit >> 5;
-  uint32_t v = __funnelshift_r(st[w], st[w + 1], bit & 31) & LIT;
-  if (order) v = __brev(v) >> 1;
-  return v;
-}
-
-// Whether local group j (global gbase + j < G) starts a stream word: a
-// literal, the first group, or a kind unlike the group before.  Threads take
-// groups j = i * WT + t in round i, so neighbouring lanes read neighbouring
-// shared-memory words.
-__device__ __forceinline__ uint32_t enc_flag(const uint32_t *st, int32_t j, uint64_t gbase, uint64_t G,
-                                             uint32_t order, uint32_t *v) {
-  *v = enc_group(st, j, order);
-  const uint32_t k = kind_of(*v);
-  // the kind of group j - 1: lane - 1 holds it; lane 0 extracts it
-  uint32_t kp = __shfl_up_sync(0xffffffffu, k, 1);
-  if ((threadIdx.x & 31) == 0) kp = kind_of(enc_group(st, j - 1, order));
-  const uint64_t g = gbase + (uint64_t)j;
-  if (g >= G) return 0u;
-  if (k == 2u || g == 0) return 1u;
-  return k != kp ? 1u : 0u;
 }
 
 // Exclusive prefix of one flag per thread over the block (lane order within
@@ -161,21 +111,8 @@ __device__ __forceinline__ uint32_t block_flag_scan(uint32_t f, uint32_t *total)
   return before + __popc(bal & ((1u << lane) - 1u));
 }
 
-// (1) stream words each block of WB groups starts.
-__global__ void __launch_bounds__(WT) wah_enc_count(const EncSrc S, uint64_t G, uint64_t *bcnt) {
-  __shared__ uint32_t st[EW + 2];
-  enc_stage(S, blockIdx.x, st);
-  const uint64_t gbase = (uint64_t)blockIdx.x * WB;
-  uint32_t c = 0, v;
-#pragma unroll
-  for (uint32_t i = 0; i < WI; ++i) c += enc_flag(st, (int32_t)(i * WT + threadIdx.x), gbase, G, S.order, &v);
-  uint64_t total;
-  block_excl_scan<uint64_t>(c, &total);
-  if (threadIdx.x == 0) bcnt[blockIdx.x] = total;
-}
-
-// (2) exclusive scan of n block values in place (one CTA, four values a
-// thread per round); v[n] = total.
+// Exclusive scan of n block values in place (one CTA, four values a thread per
+// round); v[n] = total.
 __global__ void __launch_bounds__(1024) wah_scan_blocks(uint64_t *v, uint64_t n) {
   __shared__ uint64_t part[32];
   __shared__ uint64_t carry;
@@ -213,30 +150,450 @@ __global__ void __launch_bounds__(1024) wah_scan_blocks(uint64_t *v, uint64_t n)
   if (threadIdx.x == 0) v[n] = carry;
 }
 
-// (3) the stream words: literals in full, fills with their kind only; each
-// word's starting group into pos.
-__global__ void __launch_bounds__(WT) wah_enc_write(const EncSrc S, uint64_t G, const uint64_t *boff, uint32_t *out,
-                                                    uint32_t *pos) {
-  __shared__ uint32_t st[EW + 2];
-  enc_stage(S, blockIdx.x, st);
-  const uint64_t gbase = (uint64_t)blockIdx.x * WB;
-  uint64_t at = boff[blockIdx.x];
-#pragma unroll 1
-  for (uint32_t i = 0; i < WI; ++i) {
-    const int32_t j = (int32_t)(i * WT + threadIdx.x);
-    uint32_t v, total;
-    const uint32_t f = enc_flag(st, j, gbase, G, S.order, &v);
-    const uint32_t ex = block_flag_scan(f, &total);
-    if (f) {
-      const uint32_t k = kind_of(v);
-      out[at + ex] = k == 2u ? v : (k == 1u ? FILL | ONES : FILL);
-      pos[at + ex] = (uint32_t)(gbase + (uint64_t)j);
+// The sum of the block values before block b: v[b] of a scanned array, else
+// added up here (block-collective, N threads).
+template <uint32_t N>
+__device__ __forceinline__ uint64_t sum_before(const uint64_t *v, uint64_t b, bool scanned) {
+  if (scanned) return v[b];
+  uint64_t s = 0, total;
+  for (uint64_t i0 = 0; i0 < b; i0 += 8 * N) {
+    uint64_t x[8];
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r) {
+      const uint64_t i = i0 + r * N + threadIdx.x;
+      x[r] = i < b ? v[i] : 0;
     }
-    at += total;
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r) s += x[r];
+  }
+  block_excl_scan<N, uint64_t>(s, &total);
+  return total;
+}
+
+// ----------------------------------------------------------------- streams
+// A stream prepared for reading by group blocks: note[b] and start[b] = the
+// stream word under group max(GB b - 1, 0) and that word's first group, for the
+// blocks that begin inside the stream; *total = the groups it stands for.
+struct StreamSrc {
+  const uint32_t *w;
+  uint64_t n;
+  const uint64_t *note;
+  const uint32_t *start;
+  const uint64_t *total;
+};
+
+// (1) group counts per block of WB stream words (word i * WT + t of the block in
+// round i: coalesced).
+__global__ void __launch_bounds__(WT) wah_dec_count(const uint32_t *wah, uint64_t n, uint64_t *bsum) {
+  const uint64_t kbase = (uint64_t)blockIdx.x * WB;
+  uint64_t c = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < WI; ++i) {
+    const uint64_t k = kbase + i * WT + threadIdx.x;
+    if (k < n) c += word_groups(__ldg(wah + k));
+  }
+  uint64_t total;
+  block_excl_scan<WT, uint64_t>(c, &total);
+  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
+}
+
+// Group blocks b in [b0, b1] have their note under word k, which starts at group
+// s.
+__device__ __forceinline__ void note_blocks(uint64_t *note, uint32_t *start, uint64_t b0, uint64_t b1, uint64_t k,
+                                            uint32_t s, uint32_t first, uint32_t step) {
+  for (uint64_t b = b0 + first; b <= b1; b += step) note[b] = k, start[b] = s;
+}
+
+// (2) every word's first group, and the notes of nblk group blocks.
+__global__ void __launch_bounds__(WT) wah_dec_note(const uint32_t *wah, uint64_t n, const uint64_t *bsum, bool scanned,
+                                                   uint64_t nblk, uint64_t *note, uint32_t *start, uint64_t *total) {
+  // counts in round order (coalesced loads), regrouped through shared memory so
+  // that each thread owns WI consecutive words: one block scan
+  __shared__ uint32_t xs[WB + WB / 32];  // padded: index i at i + i / 32
+  __shared__ uint64_t long_b0[GLONG], long_b1[GLONG], long_k[GLONG];
+  __shared__ uint32_t long_s[GLONG], nlong;
+  const uint64_t kbase = (uint64_t)blockIdx.x * WB;
+  if (threadIdx.x == 0) nlong = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < WI; ++i) {
+    const uint32_t l = i * WT + threadIdx.x;
+    xs[l + l / 32] = kbase + l < n ? (uint32_t)word_groups(__ldg(wah + kbase + l)) : 0u;
+  }
+  const uint64_t before = sum_before<WT>(bsum, blockIdx.x, scanned);  // (synchronises)
+  __syncthreads();
+  uint64_t sum = 0, all;
+#pragma unroll
+  for (uint32_t i = 0; i < WI; ++i) {
+    const uint32_t l = threadIdx.x * WI + i;
+    sum += xs[l + l / 32];
+  }
+  uint64_t at = before + block_excl_scan<WT, uint64_t>(sum, &all);
+  if (threadIdx.x == 0 && kbase + WB >= n) *total = before + all;
+  // (most threads' words reach no new group block)
+  const bool none = at != 0 && (at / GB == (at + sum) / GB || at / GB >= nblk);
+#pragma unroll 1
+  for (uint32_t i = 0; i < WI && !none; ++i) {
+    const uint32_t l = threadIdx.x * WI + i, ci = xs[l + l / 32];
+    const uint64_t s = at, e = at + ci, k = kbase + l;
+    at = e;
+    if (ci == 0 || s / GB >= nblk) continue;
+    // blocks b >= 1 with s <= GB b - 1 < e, and block 0 under the first group
+    const uint64_t b0 = s == 0 ? 0 : s / GB + 1, b1 = e / GB < nblk ? e / GB : nblk - 1;
+    if (b0 > b1) continue;
+    if (b1 - b0 < 8) {
+      note_blocks(note, start, b0, b1, k, (uint32_t)s, 0, 1);
+    } else {
+      const uint32_t r = atomicAdd(&nlong, 1u);
+      if (r < GLONG) long_b0[r] = b0, long_b1[r] = b1, long_k[r] = k, long_s[r] = (uint32_t)s;
+      else note_blocks(note, start, b0, b1, k, (uint32_t)s, 0, 1);
+    }
+  }
+  __syncthreads();
+  const uint32_t nl = nlong < GLONG ? nlong : GLONG;
+  for (uint32_t r = 0; r < nl; ++r) note_blocks(note, start, long_b0[r], long_b1[r], long_k[r], long_s[r], threadIdx.x, WT);
+}
+
+// Index of group-block entry x (0: the group before the block, 1 + j: its group
+// j) and of stream word x in shared memory, padded so that threads 32 apart hit
+// different banks.
+__device__ __forceinline__ uint32_t gpad(uint32_t x) { return x + (x >> 5); }
+constexpr uint32_t GPAD = GB + 1 + (GB + 1) / 32 + 1;
+
+// Entries [at, e) of a group block get value x: a short run by its lane, a long
+// one through the block's list (LongRuns), filled by all threads together.
+struct LongRuns {
+  uint32_t lo[GLONG], hi[GLONG], v[GLONG], n;
+};
+__device__ __forceinline__ void place_run(uint32_t *grp, LongRuns &R, uint32_t at, uint32_t e, uint32_t x) {
+  if (!x || at >= e) return;
+  if (e - at <= 32) {
+    for (uint32_t j = at; j < e; ++j) grp[gpad(j)] = x;
+    return;
+  }
+  const uint32_t r = atomicAdd(&R.n, 1u);
+  if (r < GLONG) R.lo[r] = at, R.hi[r] = e, R.v[r] = x;
+  else
+    for (uint32_t j = at; j < e; ++j) grp[gpad(j)] = x;
+}
+
+// The groups of block b (entry 1 + j: group GB b + j; entry 0: the group before)
+// expanded from stream T into grp; groups past the stream are 0.  Each warp takes
+// a quarter of the block's words, 32 a round: one pass for the quarters' first
+// entries, one that places the words, in which a round of one-group words only
+// needs no scan.  (Rounds unrolled with their words kept in registers ran 1.6x
+// longer: the code outgrew the instruction cache.)  Block-collective (GT threads),
+// ends synchronised.
+__device__ __forceinline__ void expand_groups(const StreamSrc &T, uint64_t b, uint64_t nblk, uint32_t order,
+                                              uint32_t *grp) {
+  constexpr uint32_t NW = GT / 32, U = 4;
+  __shared__ LongRuns R;
+  __shared__ uint32_t wsum[NW];
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (uint32_t i = t; i < GPAD; i += GT) grp[i] = 0;
+  const uint64_t total = T.n ? *T.total : 0, g0 = b ? b * GB - 1 : 0, gend = (b + 1) * GB;
+  if (g0 >= total) {
+    __syncthreads();
+    return;
+  }
+  const uint64_t k0 = T.note[b], k1 = gend <= total && b + 1 < nblk ? T.note[b + 1] : T.n - 1;
+  const uint32_t skip = (uint32_t)(g0 - T.start[b]);  // groups of the first word before g0
+  uint32_t at0 = b ? 0u : 1u;                         // entry of the next word (group g0's at first)
+  for (uint64_t kc = k0; kc <= k1 && at0 <= GB; kc += GB) {
+    const uint32_t m = k1 - kc + 1 < GB ? (uint32_t)(k1 - kc + 1) : GB;
+    const uint32_t rounds = (m + GT - 1) / GT, i0 = warp * rounds * 32 + lane;  // the lane's words: i0 + 32 r
+    const uint32_t *w = T.w + kc;
+    if (t == 0) R.n = 0;
+    auto load = [&](uint32_t r) -> uint32_t {  // past the words: a fill of no group
+      return r < rounds && i0 + 32 * r < m ? __ldg(w + i0 + 32 * r) : FILL;
+    };
+    // entries a word fills; the first word's part before g0 is left out, and no
+    // word counts for more than the block has
+    auto fills = [&](uint32_t x, uint32_t r) -> uint32_t {
+      uint32_t c = (x & FILL) ? x & CNT : 1u;
+      if (kc == k0 && i0 + 32 * r == 0) c -= skip;
+      return c < GB + 1 ? c : GB + 1;
+    };
+    uint32_t sum = 0;
+    for (uint32_t r = 0; r < rounds; r += 2 * U) {
+      uint32_t x[2 * U];
+#pragma unroll
+      for (uint32_t u = 0; u < 2 * U; ++u) x[u] = load(r + u);
+#pragma unroll
+      for (uint32_t u = 0; u < 2 * U; ++u) sum += fills(x[u], r + u);
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) wsum[warp] = sum;
+    __syncthreads();
+    uint32_t at = at0, all = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < NW; ++k) {
+      if (k < warp) at += wsum[k];
+      all += wsum[k];
+    }
+    uint32_t x[U];
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) x[u] = load(u);
+#pragma unroll 1
+    for (uint32_t r = 0; r < rounds && at <= GB; r += U) {
+      uint32_t y[U];  // the next words meanwhile
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) y[u] = load(r + U + u);
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        const uint32_t c = fills(x[u], r + u), v = group_value(x[u], order);
+        if (__all_sync(0xffffffffu, c == 1)) {
+          if (at + lane <= GB) grp[gpad(at + lane)] = v;
+          at += 32;
+          continue;
+        }
+        uint32_t inc = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const uint32_t z = __shfl_up_sync(0xffffffffu, inc, d);
+          if (lane >= (uint32_t)d) inc += z;
+        }
+        const uint32_t from = at + inc - c;
+        if (c == 1) {
+          if (from <= GB) grp[gpad(from)] = v;
+        } else {
+          place_run(grp, R, from, at + inc < GB + 1 ? at + inc : GB + 1, v);
+        }
+        at += __shfl_sync(0xffffffffu, inc, 31);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) x[u] = y[u];
+    }
+    at0 = at0 + all < GB + 1 ? at0 + all : GB + 1;
+    __syncthreads();
+    const uint32_t nl = R.n < GLONG ? R.n : GLONG;
+    for (uint32_t r = 0; r < nl; ++r)
+      for (uint32_t j = R.lo[r] + t; j < R.hi[r]; j += GT) grp[gpad(j)] = R.v[r];
+    __syncthreads();
   }
 }
 
-// (4) fill runs.
+// (3) the bitmap words of group block blockIdx.x: thread t composes words 31 t ..
+// 31 t + 30 of the block from its 32 groups.
+__global__ void __launch_bounds__(GT) wah_dec_emit(const StreamSrc T, uint64_t nblk, uint32_t order, uint64_t nrows,
+                                                   uint64_t nw, uint64_t stride, uint32_t *bm) {
+  __shared__ uint32_t grp[GPAD];
+  const uint32_t t = threadIdx.x;
+  const uint64_t b = blockIdx.x, wbase = b * GW;
+  expand_groups(T, b, nblk, order, grp);
+  uint32_t v[32];
+#pragma unroll
+  for (uint32_t j = 0; j < 32; ++j) v[j] = grp[gpad(1 + 32 * t + j)];
+  __syncthreads();
+#pragma unroll
+  for (uint32_t i = 0; i < 31; ++i) grp[31 * t + i] = (v[i] >> i) | (v[i + 1] << (31 - i));
+  __syncthreads();
+  for (uint32_t l = t; l < GW; l += GT) {
+    const uint64_t w = wbase + l;
+    if (w >= stride) break;
+    uint32_t o = w < nw ? grp[l] : 0u;
+    if (w < nw && 32 * w + 32 > nrows) o &= (1u << (nrows - 32 * w)) - 1u;
+    bm[w] = o;
+  }
+}
+
+// ------------------------------------------------------------------ encode
+// The groups to compress: a bitmap's, or op(a, b) over two streams' (0 AND, 1 OR,
+// 2 XOR).
+struct EncSrc {
+  const uint32_t *bm;  // the bitmap (NULL: the streams)
+  uint64_t nrows, nw;  // its rows and words
+  StreamSrc a, b;
+  uint32_t *groups;    // the streams' combined groups: written by the counting pass, read by the writing one
+  uint32_t op, order;
+  uint64_t G, nblk;    // groups, group blocks
+};
+enum { SRC_BITMAP = 0, SRC_STREAMS = 1, SRC_GROUPS = 2 };
+
+// The 32 groups of thread t of block b into v, and the group before them.
+// Block-collective; s0: GPAD words of shared memory.
+template <int SRC>
+__device__ __forceinline__ uint32_t enc_groups(const EncSrc &S, uint64_t b, uint32_t (&v)[32], uint32_t *s0) {
+  const uint32_t t = threadIdx.x;
+  if constexpr (SRC == SRC_GROUPS) {
+    const uint32_t *g = S.groups + b * GB + t;  // group j of thread t at j GT + t
+#pragma unroll
+    for (uint32_t j = 0; j < 32; ++j) v[j] = __ldg(g + j * GT);
+    return t ? __ldg(g + 31 * GT - 1) : b ? __ldg(g - 1) : 0u;
+  } else if constexpr (SRC == SRC_BITMAP) {
+    // s0[4 + i] = word i of the block, s0[3] the word before; every load issued
+    // before the first store
+    const uint64_t base = b * GW;
+    if (base + GW < S.nw && (reinterpret_cast<uintptr_t>(S.bm) & 15) == 0) {
+      constexpr uint32_t Q = GW / 4, R = (Q + GT - 1) / GT;  // 16-byte pieces
+      uint4 x[R];
+#pragma unroll
+      for (uint32_t r = 0; r < R; ++r)
+        if (r * GT + t < Q) x[r] = __ldg(reinterpret_cast<const uint4 *>(S.bm + base) + r * GT + t);
+      if (t == 0) s0[3] = b ? __ldg(S.bm + base - 1) : 0u;
+#pragma unroll
+      for (uint32_t r = 0; r < R; ++r)
+        if (r * GT + t < Q) reinterpret_cast<uint4 *>(s0 + 4)[r * GT + t] = x[r];
+    } else {
+      uint32_t x[31];
+#pragma unroll
+      for (uint32_t r = 0; r < 31; ++r) {
+        const uint64_t w = base + r * GT + t;
+        x[r] = w < S.nw ? __ldg(S.bm + w) : 0u;
+        if (w < S.nw && w * 32 + 32 > S.nrows) x[r] &= (1u << (S.nrows - w * 32)) - 1u;
+      }
+      if (t == 0) s0[3] = b ? __ldg(S.bm + base - 1) : 0u;
+#pragma unroll
+      for (uint32_t r = 0; r < 31; ++r) s0[4 + r * GT + t] = x[r];
+    }
+    __syncthreads();
+    // groups 32 t + j: bits 31 j .. 31 j + 30 of the thread's 31 words
+    const uint32_t *w = s0 + 4 + 31 * t;
+    uint32_t prev = w[-1] >> 1, lo = w[0];
+    v[0] = lo & LIT;
+#pragma unroll
+    for (uint32_t j = 1; j < 31; ++j) {
+      const uint32_t hi = w[j];
+      v[j] = __funnelshift_r(lo, hi, 32 - j) & LIT;
+      lo = hi;
+    }
+    v[31] = lo >> 1;
+    if (S.order) {
+#pragma unroll
+      for (uint32_t j = 0; j < 32; ++j) v[j] = __brev(v[j]) >> 1;
+      prev = __brev(prev) >> 1;
+    }
+    return prev;
+  } else {
+    expand_groups(S.a, b, S.nblk, 0, s0);
+    uint32_t prev = s0[gpad(32 * t)];
+#pragma unroll
+    for (uint32_t j = 0; j < 32; ++j) v[j] = s0[gpad(1 + 32 * t + j)];
+    __syncthreads();
+    expand_groups(S.b, b, S.nblk, 0, s0);
+    const uint32_t q = s0[gpad(32 * t)];
+    prev = S.op == 0 ? prev & q : S.op == 1 ? prev | q : prev ^ q;
+#pragma unroll
+    for (uint32_t j = 0; j < 32; ++j) {
+      const uint32_t x = s0[gpad(1 + 32 * t + j)];
+      v[j] = S.op == 0 ? v[j] & x : S.op == 1 ? v[j] | x : v[j] ^ x;
+      S.groups[b * GB + j * GT + t] = v[j];
+    }
+    return prev;
+  }
+}
+
+// Which of a thread's valid groups (bits of `valid`) are literals, and which start
+// a stream word: a literal, the table's first group, or a kind unlike the group
+// before.
+struct GroupMasks {
+  uint32_t lit, ones, start;
+};
+__device__ __forceinline__ GroupMasks group_masks(const uint32_t (&v)[32], uint32_t prev, uint32_t valid, bool first) {
+  uint32_t z = 0, o = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < 32; ++j) {
+    z |= (v[j] == 0 ? 1u : 0u) << j;
+    o |= (v[j] == LIT ? 1u : 0u) << j;
+  }
+  GroupMasks M;
+  M.lit = ~(z | o) & valid;
+  M.ones = o;
+  M.start = (M.lit | (z & ~(z << 1 | (prev == 0 ? 1u : 0u))) | (o & ~(o << 1 | (prev == LIT ? 1u : 0u))) |
+             (first ? 1u : 0u)) & valid;
+  return M;
+}
+
+__device__ __forceinline__ uint32_t valid_groups(const EncSrc &S, uint64_t b, uint32_t t) {  // of thread t: 0 .. 32
+  const uint64_t g = b * GB + 32ull * t;
+  return g >= S.G ? 0u : S.G - g < 32 ? (uint32_t)(S.G - g) : 32u;
+}
+
+// (1) stream words each block starts.
+template <int SRC>
+__global__ void __launch_bounds__(GT) wah_enc_count(const __grid_constant__ EncSrc S, uint64_t *bcnt) {
+  __shared__ __align__(16) uint32_t s0[GPAD];
+  const uint64_t b = blockIdx.x;
+  uint32_t v[32];
+  const uint32_t prev = enc_groups<SRC>(S, b, v, s0);
+  const uint32_t nv = valid_groups(S, b, threadIdx.x);
+  const GroupMasks M = group_masks(v, prev, nv == 32 ? 0xffffffffu : (1u << nv) - 1u, b == 0 && threadIdx.x == 0);
+  uint32_t total;
+  block_excl_scan<GT, uint32_t>(__popc(M.start), &total);
+  if (threadIdx.x == 0) bcnt[b] = total;
+}
+
+// (2) the stream words, in order: literals, and fills with the part of their run
+// that lies in the block.  off[b] = the block's first word, cont[b] = its groups
+// that continue the run before it; *nwords = the stream's words.
+template <int SRC>
+__global__ void __launch_bounds__(GT, 7) wah_enc_write(const __grid_constant__ EncSrc S, const uint64_t *bcnt,
+                                                    bool scanned, uint32_t *out, uint64_t *off, uint32_t *cont,
+                                                    uint64_t *nwords) {
+  __shared__ __align__(16) uint32_t s0[GPAD];
+  __shared__ uint32_t wfirst[GT / 32];  // per warp: groups before its first start (all its groups if none)
+  __shared__ uint32_t whas[GT / 32];
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint64_t b = blockIdx.x;
+  uint32_t v[32];
+  const uint32_t prev = enc_groups<SRC>(S, b, v, s0);
+  const uint32_t nv = valid_groups(S, b, t);
+  const GroupMasks M = group_masks(v, prev, nv == 32 ? 0xffffffffu : (1u << nv) - 1u, b == 0 && t == 0);
+  const uint64_t at = sum_before<GT>(bcnt, b, scanned);  // 
+  uint32_t total;
+  uint32_t pos = block_excl_scan<GT, uint32_t>(__popc(M.start), &total);
+  // groups from the end of the thread's to the next start, or to the block's end
+  const uint32_t first = M.start ? (uint32_t)__ffs(M.start) - 1 : nv;
+  const uint32_t has = __ballot_sync(0xffffffffu, M.start != 0);
+  const uint32_t wgroups = __reduce_add_sync(0xffffffffu, nv);
+  const uint32_t fl = has ? (uint32_t)__ffs(has) - 1 : 0u, ff = __shfl_sync(0xffffffffu, first, fl);
+  if (lane == 0) wfirst[warp] = has ? 32 * fl + ff : wgroups, whas[warp] = has ? 1u : 0u;
+  __syncthreads();
+  const uint32_t later = lane == 31 ? 0u : has & (0xffffffffu << (lane + 1));
+  const uint32_t nl = later ? (uint32_t)__ffs(later) - 1 : lane, nf = __shfl_sync(0xffffffffu, first, nl);
+  uint32_t dist;
+  if (later) {
+    dist = 32 * (nl - lane - 1) + nf;
+  } else {
+    dist = wgroups > 32 * (lane + 1) ? wgroups - 32 * (lane + 1) : 0u;
+    for (uint32_t w = warp + 1; w < GT / 32; ++w) {
+      dist += wfirst[w];
+      if (whas[w]) break;
+    }
+  }
+  if (t == 0) {
+    uint32_t c = 0;
+    for (uint32_t w = 0; w < GT / 32; ++w) {
+      c += wfirst[w];
+      if (whas[w]) break;
+    }
+    off[b] = at;
+    cont[b] = c;
+    if (b + 1 == S.nblk) *nwords = at + total;
+  }
+  // the words into s0 (at most GB), then out
+#pragma unroll
+  for (uint32_t j = 0; j < 32; ++j)
+    if ((M.start >> j) & 1u) {
+      uint32_t w = v[j];
+      if (!((M.lit >> j) & 1u)) {
+        const uint32_t rest = M.start >> j >> 1;
+        const uint32_t run = rest ? (uint32_t)__ffs(rest) : nv - j + dist;
+        w = FILL | ((M.ones >> j) & 1u ? ONES : 0u) | run;
+      }
+      s0[pos++] = w;
+    }
+  __syncthreads();
+  for (uint32_t i = t; i < total; i += GT) out[at + i] = s0[i];
+}
+
+// (3) a block's groups before its first start belong to the last fill before it.
+__global__ void wah_enc_join(uint32_t *out, const uint64_t *off, const uint32_t *cont, uint64_t nblk) {
+  const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b == 0 || b >= nblk) return;
+  if (cont[b]) atomicAdd(&out[off[b] - 1], cont[b]);
+}
+
+// (direct) fill runs.
 __global__ void wah_enc_fills(uint32_t *out, const uint32_t *pos, uint64_t K, uint64_t G) {
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < K; k += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t w = out[k];
@@ -247,26 +604,19 @@ __global__ void wah_enc_fills(uint32_t *out, const uint32_t *pos, uint64_t K, ui
   }
 }
 
-__device__ __forceinline__ uint64_t word_groups(uint32_t w) { return (w & FILL) ? (w & CNT) : 1u; }
-
-// decode (1): group counts per block of WB stream words (word i * WT + t of
-// the block in round i: coalesced).
-__global__ void __launch_bounds__(WT) wah_dec_count(const uint32_t *wah, uint64_t n, uint64_t *bsum) {
-  const uint64_t kbase = (uint64_t)blockIdx.x * WB;
-  uint64_t c = 0;
-#pragma unroll
-  for (uint32_t i = 0; i < WI; ++i) {
-    const uint64_t k = kbase + i * WT + threadIdx.x;
-    if (k < n) c += word_groups(__ldg(wah + k));
+// Largest k in [lo, hi] with S[k] <= g (S ascending, S[lo] <= g).
+__device__ __forceinline__ uint64_t last_le(const uint32_t *S, uint64_t lo, uint64_t hi, uint64_t g) {
+  while (lo < hi) {
+    const uint64_t mid = lo + (hi - lo + 1) / 2;
+    if (S[mid] <= g) lo = mid;
+    else hi = mid - 1;
   }
-  uint64_t total;
-  block_excl_scan<uint64_t>(c, &total);
-  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
+  return lo;
 }
 
-// decode (2b): the exclusive scan of every word's group count; S[n] = total.
-// S is stored saturated at 2^32 - 1: decoding looks up groups below 2^30
-// only, and min(x, cap) keeps the order of every prefix below the cap.
+// (direct) the exclusive scan of every word's group count; S[n] = total.
+// S is stored saturated at 2^32 - 1: lookups are of groups below 2^30 only, and
+// min(x, cap) keeps the order of every prefix below the cap.
 __device__ __forceinline__ uint32_t sat32(uint64_t x) { return x > 0xffffffffull ? 0xffffffffu : (uint32_t)x; }
 
 __global__ void __launch_bounds__(WT) wah_dec_scan(const uint32_t *wah, uint64_t n, const uint64_t *boff,
@@ -295,7 +645,7 @@ __global__ void __launch_bounds__(WT) wah_dec_scan(const uint32_t *wah, uint64_t
     sum += c[i];
   }
   uint64_t total;
-  uint64_t at = boff[blockIdx.x] + block_excl_scan<uint64_t>(sum, &total);
+  uint64_t at = boff[blockIdx.x] + block_excl_scan<WT, uint64_t>(sum, &total);
 #pragma unroll
   for (uint32_t i = 0; i < WI; ++i) {
     const uint32_t l = threadIdx.x * WI + i;
@@ -312,158 +662,116 @@ __global__ void __launch_bounds__(WT) wah_dec_scan(const uint32_t *wah, uint64_t
   if (blockIdx.x == 0 && threadIdx.x == 0) S[n] = sat32(boff[nblk]);
 }
 
-// Largest k in [lo, hi] with S[k] <= g (S ascending, S[lo] <= g).
-__device__ __forceinline__ uint64_t last_le(const uint32_t *S, uint64_t lo, uint64_t hi, uint64_t g) {
-  while (lo < hi) {
-    const uint64_t mid = lo + (hi - lo + 1) / 2;
-    if (S[mid] <= g) lo = mid;
-    else hi = mid - 1;
+// A pinned host word per thread that kernels write a result to.
+struct HostWord {
+  uint64_t *p = nullptr;
+  ~HostWord() {
+    if (p) cudaFreeHost(p);
   }
-  return lo;
+};
+mb_status host_word(uint64_t **out) {
+  static thread_local HostWord w;
+  if (!w.p) MB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&w.p), sizeof(uint64_t), cudaHostAllocPortable | cudaHostAllocMapped));
+  *out = w.p;
+  return MB_OK;
 }
 
-// decode (3): for output block b (words [DW b, DW (b + 1))), the stream
-// words covering its groups.
-__global__ void wah_dec_partition(const uint32_t *S, uint64_t n, uint64_t nblk, uint64_t *kb, uint64_t *ke) {
-  const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nblk) return;
-  const uint64_t total = S[n];
-  const uint64_t w0 = b * DW, w1 = w0 + DW - 1;
-  const uint64_t ga = (32 * w0) / 31, gz = (32 * w1) / 31 + 1;
-  if (ga >= total) {
-    kb[b] = 1, ke[b] = 0;  // past the stream: an empty range
-    return;
+// A call's scratch: one allocation, carved into 16-byte aligned pieces (an
+// allocation and its release cost the host 3-4 us a pair).
+struct Carve {
+  uint8_t *base = nullptr;
+  size_t used = 0;  // counted without a base, handed out with one
+  template <typename T>
+  T *take(uint64_t n) {
+    T *p = reinterpret_cast<T *>(base ? base + used : nullptr);
+    used += round_up(std::max<uint64_t>(n, 1) * sizeof(T), 16);
+    return p;
   }
-  const uint64_t s = last_le(S, 0, n - 1, ga);
-  kb[b] = s;
-  ke[b] = last_le(S, s, n - 1, gz < total ? gz : total - 1);
+};
+// Runs `plan` twice: to count the bytes, then with them allocated.
+template <typename F>
+mb_status carve(Scratch &sc, F plan) {
+  Carve c;
+  plan(c);
+  MB_CHECK(sc.get(&c.base, c.used));
+  c.used = 0;
+  plan(c);
+  return MB_OK;
 }
 
-__device__ __forceinline__ uint32_t group_value(uint32_t word, uint32_t order) {
-  uint32_t x = (word & FILL) ? ((word & ONES) ? LIT : 0u) : (word & LIT);
-  return order ? __brev(x) >> 1 : x;
+// Block values v[0 .. n) ready for sum_before: scanned when there are many, or
+// when the caller needs the total in v[n].
+mb_status block_sums(uint64_t *v, uint64_t n, bool total, bool *scanned, cudaStream_t st) {
+  *scanned = total || n > DIRECT_SUM;
+  if (!*scanned) return MB_OK;
+  wah_scan_blocks<<<1, 1024, 0, st>>>(v, n);
+  MB_LAUNCH_CHECK("wah_scan_blocks");
+  return MB_OK;
 }
 
-// decode (4): the block expands its staged stream words into its groups in
-// shared memory (0 groups are the default; runs longer than 32 groups are
-// filled by all threads together), then each thread composes output words
-// w = DW b + i DT + t from the two groups each spans.
-__global__ void __launch_bounds__(DT) wah_dec_emit(const uint32_t *wah, const uint32_t *S, uint64_t n,
-                                                   const uint64_t *kb, const uint64_t *ke, uint32_t order,
-                                                   uint64_t nrows, uint64_t nw, uint64_t stride, uint32_t *bm) {
-  __shared__ uint32_t s_S[DCAP + 1];
-  __shared__ uint32_t s_w[DCAP];
-  __shared__ uint32_t grp[DGRP];
-  __shared__ uint32_t long_lo[DLONG], long_hi[DLONG], long_v[DLONG];
-  __shared__ uint32_t nlong;
-  const uint32_t t = threadIdx.x;
-  const uint64_t b = blockIdx.x, wbase = b * DW;
-  const uint64_t ga0 = (32 * wbase) / 31;
-  const uint64_t lo = kb[b], hi = ke[b], total = S[n];
-  const bool empty = lo > hi, staged = !empty && hi - lo + 1 <= DCAP;
-  const uint32_t cnt = staged ? (uint32_t)(hi - lo + 1) : 0u;
-  const uint64_t wend = wbase + DW < nw ? wbase + DW : nw;
-  const uint32_t ng = wend > wbase ? (uint32_t)((32 * (wend - 1)) / 31 + 2 - ga0) : 0u;
-  const uint64_t gcap = ga0 + ng < total ? ga0 + ng : total;  // groups with a value: [ga0, gcap)
-  for (uint32_t j = t; j < ng; j += DT) grp[j] = 0;
-  if (t == 0) nlong = 0;
-  if (staged) {
-    constexpr uint32_t R = (DCAP + DT - 1) / DT;
-    uint32_t a[R], c[R];
-#pragma unroll
-    for (uint32_t r = 0; r < R; ++r) {  // every load issued before the first store
-      const uint32_t i = r * DT + t;
-      if (i < cnt) a[r] = S[lo + i], c[r] = __ldg(wah + lo + i);
-    }
-#pragma unroll
-    for (uint32_t r = 0; r < R; ++r) {
-      const uint32_t i = r * DT + t;
-      if (i < cnt) s_S[i] = a[r], s_w[i] = c[r];
-    }
-    if (t == 0) s_S[cnt] = S[hi + 1];
+// Scratch of an encoding of nblk group blocks, and of a stream's notes for them.
+struct EncBufs {
+  uint64_t *bcnt, *off;
+  uint32_t *cont, *groups;
+  void plan(Carve &c, uint64_t nblk, bool streams) {
+    groups = streams ? c.take<uint32_t>(nblk * GB) : nullptr;
+    bcnt = c.take<uint64_t>(nblk + 1), off = c.take<uint64_t>(nblk), cont = c.take<uint32_t>(nblk);
   }
-  __syncthreads();
-  if (staged) {
-    // local group range of the block: [0, lcap); S values are < 2^32 here
-    const uint32_t g_lo = (uint32_t)ga0, lcap = (uint32_t)(gcap > ga0 ? gcap - ga0 : 0);
-    for (uint32_t i = t; i < cnt; i += DT) {
-      const uint32_t x = group_value(s_w[i], order);
-      if (!x) continue;
-      const uint32_t a = s_S[i] > g_lo ? s_S[i] - g_lo : 0u, e0 = s_S[i + 1] > g_lo ? s_S[i + 1] - g_lo : 0u;
-      const uint32_t e = e0 < lcap ? e0 : lcap;
-      if (a >= e) continue;
-      if (e - a <= 32) {
-        for (uint32_t j = a; j < e; ++j) grp[j] = x;
-      } else {
-        const uint32_t r = atomicAdd(&nlong, 1u);
-        if (r < DLONG) long_lo[r] = a, long_hi[r] = e, long_v[r] = x;
-        else
-          for (uint32_t j = a; j < e; ++j) grp[j] = x;
-      }
-    }
+};
+struct NoteBufs {
+  uint64_t *bsum, *note;
+  uint32_t *start;
+  void plan(Carve &c, uint64_t n, uint64_t nblk) {
+    bsum = c.take<uint64_t>(ceil_div(n, WB) + 2), note = c.take<uint64_t>(nblk), start = c.take<uint32_t>(nblk);
   }
-  __syncthreads();
-  const uint32_t nl = nlong < DLONG ? nlong : DLONG;
-  for (uint32_t r = 0; r < nl; ++r)
-    for (uint32_t j = long_lo[r] + t; j < long_hi[r]; j += DT) grp[j] = long_v[r];
-  __syncthreads();
-  // word wbase + l holds rows from local group (rb + 32 l) / 31 at bit
-  // (rb + 32 l) % 31 on, rb = 32 wbase - 31 ga0 (< 31): 32-bit arithmetic
-  const uint32_t rb = (uint32_t)(32 * wbase - 31 * ga0);
-#pragma unroll 1
-  for (uint32_t i = 0; i < DV; ++i) {
-    const uint32_t l = i * DT + t;
-    const uint64_t w = wbase + l;
-    if (w >= stride) break;
-    uint32_t o = 0;
-    if (!empty && w < nw) {
-      const uint32_t q = rb + 32 * l, la = q / 31, sa = q - 31 * la;
-      uint32_t va, vb;
-      if (staged) {
-        va = grp[la];
-        vb = grp[la + 1];
-      } else {  // more stream words than the stage holds (runs of 0 groups): search
-        const uint64_t ga = ga0 + la;
-        va = ga < total ? group_value(__ldg(wah + last_le(S, lo, hi, ga)), order) : 0u;
-        vb = ga + 1 < total ? group_value(__ldg(wah + last_le(S, lo, hi, ga + 1)), order) : 0u;
-      }
-      o = (va >> sa) | (vb << (31 - sa));
-      const uint64_t r0 = 32 * w;
-      if (r0 + 32 > nrows) o &= nrows > r0 ? (1u << (nrows - r0)) - 1u : 0u;
-    }
-    bm[w] = o;
-  }
-}
+};
 
 // Encodes the groups of S into out (capacity words); *nwords = words of the
 // stream, also when it does not fit (nothing is written then).
-mb_status encode(const EncSrc &S, uint32_t *out, uint64_t capacity, uint64_t *nwords, cudaStream_t st,
-                 const char *who) {
-  const uint64_t G = ceil_div(S.nrows, 31);
-  *nwords = 0;
-  if (G == 0) return MB_OK;
-  const uint64_t nblk = ceil_div(G, WB);
-  Scratch sc(st);
-  uint64_t *boff;
-  MB_CHECK(sc.get(&boff, nblk + 1));
-  wah_enc_count<<<(unsigned)nblk, WT, 0, st>>>(S, G, boff);
+template <int SRC>
+mb_status encode(const EncSrc &S, const EncBufs &B, uint32_t *out, uint64_t capacity, uint64_t *nwords,
+                 cudaStream_t st, const char *who) {
+  const unsigned grid = (unsigned)S.nblk;
+  uint64_t *hw;
+  MB_CHECK(host_word(&hw));
+  wah_enc_count<SRC><<<grid, GT, 0, st>>>(S, B.bcnt);
   MB_LAUNCH_CHECK("wah_enc_count");
-  wah_scan_blocks<<<1, 1024, 0, st>>>(boff, nblk);
-  MB_LAUNCH_CHECK("wah_scan_blocks");
-  uint64_t K = 0;
-  MB_CUDA(cudaMemcpyAsync(&K, boff + nblk, 8, cudaMemcpyDeviceToHost, st));
-  MB_CUDA(cudaStreamSynchronize(st));
-  *nwords = K;
-  if (!out) return MB_OK;  // a size query
-  if (K > capacity) return fail(MB_ERR_INVALID, "%s: the stream has %llu words, the output holds %llu", who,
-                                (unsigned long long)K, (unsigned long long)capacity);
-  uint32_t *pos;
-  MB_CHECK(sc.get(&pos, K));
-  wah_enc_write<<<(unsigned)nblk, WT, 0, st>>>(S, G, boff, out, pos);
+  // a stream has at most a word a group: only a smaller output needs the size first
+  const bool sized = !out || capacity < S.G;
+  bool scanned = false;
+  MB_CHECK(block_sums(B.bcnt, S.nblk, sized, &scanned, st));
+  if (sized) {
+    MB_CUDA(cudaMemcpyAsync(hw, B.bcnt + S.nblk, 8, cudaMemcpyDeviceToHost, st));
+    MB_CUDA(cudaStreamSynchronize(st));
+    *nwords = *hw;
+    if (!out) return MB_OK;  // a size query
+    if (*nwords > capacity) return fail(MB_ERR_INVALID, "%s: the stream has %llu words, the output holds %llu", who,
+                                        (unsigned long long)*nwords, (unsigned long long)capacity);
+  }
+  wah_enc_write<SRC == SRC_STREAMS ? SRC_GROUPS : SRC><<<grid, GT, 0, st>>>(S, B.bcnt, scanned, out, B.off, B.cont, hw);
   MB_LAUNCH_CHECK("wah_enc_write");
-  const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(K, 256), (uint64_t)dev_info().sms * 8);
-  wah_enc_fills<<<grid, 256, 0, st>>>(out, pos, K, G);
-  MB_LAUNCH_CHECK("wah_enc_fills");
+  if (S.nblk > 1) {
+    wah_enc_join<<<(unsigned)ceil_div(S.nblk, 256), 256, 0, st>>>(out, B.off, B.cont, S.nblk);
+    MB_LAUNCH_CHECK("wah_enc_join");
+  }
+  MB_CUDA(cudaStreamSynchronize(st));  // *hw
+  *nwords = *hw;
+  return MB_OK;
+}
+
+// The notes of stream (wah, n) for nblk group blocks.
+mb_status prepare_stream(const uint32_t *wah, uint64_t n, uint64_t nblk, const NoteBufs &B, StreamSrc *T,
+                         cudaStream_t st) {
+  *T = StreamSrc{wah, n, nullptr, nullptr, nullptr};
+  if (n == 0) return MB_OK;
+  const uint64_t sblk = ceil_div(n, WB);
+  wah_dec_count<<<(unsigned)sblk, WT, 0, st>>>(wah, n, B.bsum);
+  MB_LAUNCH_CHECK("wah_dec_count");
+  bool scanned = false;
+  MB_CHECK(block_sums(B.bsum, sblk, false, &scanned, st));
+  wah_dec_note<<<(unsigned)sblk, WT, 0, st>>>(wah, n, B.bsum, scanned, nblk, B.note, B.start, B.bsum + sblk + 1);
+  MB_LAUNCH_CHECK("wah_dec_note");
+  T->note = B.note, T->start = B.start, T->total = B.bsum + sblk + 1;
   return MB_OK;
 }
 
@@ -493,15 +801,12 @@ mb_status decode(const uint32_t *wah, uint64_t n, uint32_t order, uint64_t nrows
     return MB_OK;
   }
   Scratch sc(st);
-  uint32_t *S;
-  MB_CHECK(group_scan(wah, n, sc, &S, st));
-  const uint64_t nblk = ceil_div(stride, DW);
-  uint64_t *kb, *ke;
-  MB_CHECK(sc.get(&kb, nblk));
-  MB_CHECK(sc.get(&ke, nblk));
-  wah_dec_partition<<<(unsigned)ceil_div(nblk, 256), 256, 0, st>>>(S, n, nblk, kb, ke);
-  MB_LAUNCH_CHECK("wah_dec_partition");
-  wah_dec_emit<<<(unsigned)nblk, DT, 0, st>>>(wah, S, n, kb, ke, order, nrows, nw, stride, bm);
+  const uint64_t nblk = ceil_div(stride, GW);
+  NoteBufs B;
+  MB_CHECK(carve(sc, [&](Carve &c) { B.plan(c, n, nblk); }));
+  StreamSrc T;
+  MB_CHECK(prepare_stream(wah, n, nblk, B, &T, st));
+  wah_dec_emit<<<(unsigned)nblk, GT, 0, st>>>(T, nblk, order, nrows, nw, stride, bm);
   MB_LAUNCH_CHECK("wah_dec_emit");
   return MB_OK;
 }
@@ -582,7 +887,7 @@ __global__ void __launch_bounds__(WT) wah_direct_count(const DirectSrc D, const 
   for (uint32_t i = 0; i < WI; ++i)
     c += direct_flag(D, m, M, (uint64_t)blockIdx.x * WB + i * WT + threadIdx.x, &v, &x) ? 1u : 0u;
   uint64_t total;
-  block_excl_scan<uint64_t>(c, &total);
+  block_excl_scan<WT, uint64_t>(c, &total);
   if (threadIdx.x == 0) bcnt[blockIdx.x] = total;
 }
 
@@ -669,8 +974,15 @@ extern "C" mb_status mb_wah_encode(const uint32_t *bitmap, uint64_t nrows, uint3
   if (ceil_div(nrows, 31) > MAX_GROUPS)
     return fail(MB_ERR_INVALID, "mb_wah_encode: %llu rows exceed the 30-bit run count", (unsigned long long)nrows);
   if (!aligned4(bitmap) || !aligned4(wah)) return fail(MB_ERR_INVALID, "mb_wah_encode: misaligned pointer");
-  const EncSrc S{bitmap, nullptr, 0, order, nrows, mb_bitmap_words(nrows)};
-  return encode(S, wah, capacity, nwords, as_stream(stream), "mb_wah_encode");
+  EncSrc S{};
+  S.bm = bitmap, S.nrows = nrows, S.nw = mb_bitmap_words(nrows), S.order = order, S.G = ceil_div(nrows, 31);
+  if (S.G == 0) return MB_OK;
+  S.nblk = ceil_div(S.G, GB);
+  cudaStream_t st = as_stream(stream);
+  Scratch sc(st);
+  EncBufs B;
+  MB_CHECK(carve(sc, [&](Carve &c) { B.plan(c, S.nblk, false); }));
+  return encode<SRC_BITMAP>(S, B, wah, capacity, nwords, st, "mb_wah_encode");
 }
 
 extern "C" mb_status mb_wah_decode(const uint32_t *wah, uint64_t nwords, uint32_t order, uint64_t nrows,
@@ -719,21 +1031,22 @@ extern "C" mb_status mb_wah_op_ex(uint32_t op, const uint32_t *a, uint64_t na, c
                                         (unsigned long long)ngroups);
   if (ngroups == 0) return MB_OK;
   cudaStream_t st = as_stream(stream);
-  // direct when the streams are short next to the groups: its work follows
-  // the words (with a binary search per piece), the explicit form's the rows
-  if (method == MB_WAH_DIRECT || (method == MB_WAH_AUTO && 8 * (na + nb) < ngroups))
+  // direct when the streams are short next to the groups: its work follows the
+  // words (with binary searches per piece), the other form's the groups
+  if (method == MB_WAH_DIRECT || (method == MB_WAH_AUTO && DIRECT_RATIO * (na + nb) < ngroups))
     return direct_op(op, a, na, b, nb, ngroups, out, capacity, nwords, st);
-  // decode both (the order is immaterial: both sides and the result keep
-  // the streams' own), then encode op(x, y)
-  const uint64_t nrows = 31 * ngroups, stride = mb_bitmap_stride(nrows);
+  // the encoder on the groups of both streams, expanded block by block (their
+  // bit order is immaterial: both sides and the result keep their own)
   Scratch sc(st);
-  uint32_t *x, *y;
-  MB_CHECK(sc.get(&x, stride));
-  MB_CHECK(sc.get(&y, stride));
-  MB_CHECK(decode(a, na, 0, nrows, x, st));
-  MB_CHECK(decode(b, nb, 0, nrows, y, st));
-  const EncSrc S{x, y, op, 0, nrows, mb_bitmap_words(nrows)};
-  return encode(S, out, capacity, nwords, st, "mb_wah_op");
+  EncSrc S{};
+  S.op = op, S.G = ngroups, S.nblk = ceil_div(ngroups, GB);
+  EncBufs B;
+  NoteBufs A1, A2;
+  MB_CHECK(carve(sc, [&](Carve &c) { B.plan(c, S.nblk, true), A1.plan(c, na, S.nblk), A2.plan(c, nb, S.nblk); }));
+  MB_CHECK(prepare_stream(a, na, S.nblk, A1, &S.a, st));
+  MB_CHECK(prepare_stream(b, nb, S.nblk, A2, &S.b, st));
+  S.groups = B.groups;
+  return encode<SRC_STREAMS>(S, B, out, capacity, nwords, st, "mb_wah_op");
 }
 
 // The reference's WAH file (struct wahHost_s, merle/host/wahCpu.h:10-15, read
