@@ -25,6 +25,7 @@
 // block in the device error word and leaves the loop block-uniformly.
 #include <string.h>
 #include "common.cuh"
+#include "opdrain.cuh"
 #include "opeval.cuh"
 #include "tma.cuh"
 #include "vbp.cuh"
@@ -46,89 +47,11 @@ OpNeeds op_needs(const mb_op &O) {
   return n;
 }
 
-__device__ __forceinline__ uint32_t ld_w32(const void *p, uint64_t i, uint32_t w) {
-  switch (w) {
-  case 1: return __ldg(reinterpret_cast<const uint8_t *>(p) + i);
-  case 2: return __ldg(reinterpret_cast<const uint16_t *>(p) + i);
-  default: return __ldg(reinterpret_cast<const uint32_t *>(p) + i);
-  }
-}
-
-// v[s] for a warp-uniform runtime s without dynamic register indexing.
-__device__ __forceinline__ uint32_t pick(const uint32_t (&v)[MB_MAXSRC], uint32_t s) {
-  uint32_t r = v[0];
-#pragma unroll
-  for (uint32_t i = 1; i < MB_MAXSRC; ++i) r = (s == i) ? v[i] : r;
-  return r;
-}
-
-// Loads every needed source of one row: foreign keys first, then values.
-// bad: bit s set if source s's key is out of its dimension.
-__device__ __forceinline__ void load_row(const mb_op &O, uint32_t need, uint32_t row, uint32_t (&v)[MB_MAXSRC],
-                                         uint32_t &bad) {
-  uint32_t key[MB_MAXSRC];
-#pragma unroll
-  for (uint32_t s = 0; s < MB_MAXSRC; ++s) {
-    key[s] = row;
-    if (s < O.nsrc && ((need >> s) & 1u) && O.src[s].fk) key[s] = __ldg(O.src[s].fk + row);
-  }
-  bad = 0;
-#pragma unroll
-  for (uint32_t s = 0; s < MB_MAXSRC; ++s) {
-    v[s] = 0;
-    if (s < O.nsrc && ((need >> s) & 1u)) {
-      const mb_src &S = O.src[s];
-      if (S.fk && S.dimsz != 0 && key[s] >= S.dimsz) bad |= 1u << s;
-      else v[s] = ld_w32(S.col, key[s], S.width);
-    }
-  }
-}
-
-// The op's filter over loaded values.
-__device__ __forceinline__ bool filter_row(const mb_op &O, const uint32_t (&v)[MB_MAXSRC], uint32_t bad) {
-  uint32_t t = 0;
-  for (uint32_t c = 0; c < O.nclause; ++c) {
-    bool any = false;
-    const uint32_t len = O.clause_len[c];
-    for (uint32_t k = 0; k < len; ++k, ++t) {
-      const mb_term &tm = O.terms[t];
-      const uint64_t x = pick(v, tm.src);
-      any |= !((bad >> tm.src) & 1u) && x >= tm.lo && x < tm.hi;
-    }
-    if (!any) return false;
-  }
-  return true;
-}
-
-// The op over loaded values (the same semantics as op_eval in opeval.cuh).
-__device__ __forceinline__ bool eval_row(const mb_op &O, const uint32_t (&v)[MB_MAXSRC], uint32_t bad, bool chk,
-                                         uint32_t nr_grp, int64_t &value, uint32_t &group) {
-  if (chk && !filter_row(O, v, bad)) return false;
-  uint32_t g = 0;
-  for (uint32_t k = 0; k < O.nkey; ++k) {
-    const mb_key &kk = O.keys[k];
-    if ((bad >> kk.src) & 1u) return false;
-    uint32_t x = pick(v, kk.src);
-    if (kk.xform == MB_X_DIV) x = x / kk.div;
-    else if (kk.xform == MB_X_YEAR) x = date_to_year(x);
-    g += kk.mul * (x - kk.base);
-  }
-  if (g >= nr_grp) return false;
-  if (O.vkind == MB_V_ONE) {
-    value = 1;
-  } else {
-    if ((bad >> O.va) & 1u) return false;
-    const uint64_t a = pick(v, O.va);
-    if (O.vkind == MB_V_COL) {
-      value = (int64_t)a;
-    } else {
-      if ((bad >> O.vb) & 1u) return false;
-      const uint64_t b = pick(v, O.vb);
-      value = O.vkind == MB_V_MUL ? (int64_t)(a * b) : (int64_t)a - (int64_t)b;
-    }
-  }
-  group = g;
-  return true;
+bool op_reads_wide(const mb_op &O) {
+  const OpNeeds n = op_needs(O);
+  for (uint32_t s = 0; s < O.nsrc; ++s)
+    if (((n.kv_mask | n.filt_mask) >> s & 1u) && O.src[s].width > 4) return true;
+  return false;
 }
 
 // Word lw of bitmap b in the staged tile; words past the bulk-copied part of
@@ -257,26 +180,6 @@ __device__ __forceinline__ void vbp_eval_staged(const DevPrg &P, const TileView 
   }
 }
 
-// Runs the op over 64 queued rows (two per lane) and aggregates them.
-template <bool CHK, int GS>
-__device__ __forceinline__ void drain64(const mb_op &O, const OpNeeds &N, const uint32_t *q, uint32_t nrows_avail,
-                                        uint32_t nr_grp, const GrpCtx &G, int64_t &acc, uint64_t &cnt) {
-  const uint32_t lane = threadIdx.x & 31;
-  const bool ok0 = lane < nrows_avail, ok1 = lane + 32 < nrows_avail;
-  const uint32_t e0 = ok0 ? q[lane] : 0u, e1 = ok1 ? q[lane + 32] : 0u;
-  const bool c0 = CHK && (e0 >> 31), c1 = CHK && (e1 >> 31);
-  uint32_t v0[MB_MAXSRC], v1[MB_MAXSRC], bad0, bad1;
-  load_row(O, ok0 ? (N.kv_mask | (c0 ? N.filt_mask : 0u)) : 0u, e0 & 0x7fffffffu, v0, bad0);
-  load_row(O, ok1 ? (N.kv_mask | (c1 ? N.filt_mask : 0u)) : 0u, e1 & 0x7fffffffu, v1, bad1);
-  int64_t val0 = 0, val1 = 0;
-  uint32_t g0 = 0, g1 = 0;
-  const bool k0 = ok0 && eval_row(O, v0, bad0, c0, nr_grp, val0, g0);
-  const bool k1 = ok1 && eval_row(O, v1, bad1, c1, nr_grp, val1, g1);
-  cnt += (k0 ? 1u : 0u) + (k1 ? 1u : 0u);
-  aggregate<GS>(G, k0, g0, val0, acc);
-  if (nrows_avail > 32) aggregate<GS>(G, k1, g1, val1, acc);
-}
-
 constexpr uint32_t FT_QCAP = 32 * 32 + 64;  // one 32-word chunk + fewer than 64 pending rows
 
 // Appends the set rows of one 32-word chunk (word w0 + lane of each lane,
@@ -286,7 +189,7 @@ constexpr uint32_t FT_QCAP = 32 * 32 + 64;  // one 32-word chunk + fewer than 64
 template <bool CHK, int GS>
 __device__ __forceinline__ void compact_chunk(const mb_op &O, const OpNeeds &N, uint32_t *queue, uint32_t &qn,
                                               uint64_t w0, uint32_t m, uint32_t uw, uint32_t nr_grp,
-                                              const GrpCtx &G, int64_t &acc, uint64_t &cnt) {
+                                              const GrpCtx &G, int64_t &acc, uint32_t &cnt) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t pc = __popc(m);
   uint32_t incl = pc;
@@ -310,7 +213,7 @@ __device__ __forceinline__ void compact_chunk(const mb_op &O, const OpNeeds &N, 
   __syncwarp();
   while (qn >= 64) {  // drain from the end: the queue's order is irrelevant
     qn -= 64;
-    drain64<CHK, GS>(O, N, queue + qn, 64, nr_grp, G, acc, cnt);
+    drain64<CHK ? DR_FLAG : DR_NOCHK, GS>(O, N, queue + qn, 64, nr_grp, G, acc, cnt);
   }
   __syncwarp();
 }
@@ -323,9 +226,7 @@ struct AnyDrain {
   uint32_t nr_grp;
   __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, bool, const GrpCtx &G, int64_t &acc,
                                         uint32_t &cnt) const {
-    uint64_t c = 0;
-    drain64<CHK, GS>(O, N, q, n, nr_grp, G, acc, c);
-    cnt += (uint32_t)c;
+    drain64<CHK ? DR_FLAG : DR_NOCHK, GS>(O, N, q, n, nr_grp, G, acc, cnt);
   }
 };
 
@@ -381,7 +282,7 @@ fused_tma_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ mb_op
   }
 
   int64_t acc = 0;
-  uint64_t cnt = 0;
+  uint32_t cnt = 0;
   uint32_t qn = 0;  // rows pending in this warp's queue (warp-uniform)
   uint32_t it = 0;
   const uint32_t nchunks = T / 32;
@@ -429,7 +330,7 @@ fused_tma_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ mb_op
       compact_chunk<CHK, GS>(O, N, queue, qn, tv.w0 + c * 32, ptile[c * 32 + lane], CHK ? utile[c * 32 + lane] : 0u,
                              nr_grp, G, acc, cnt);
   }
-  if (qn) drain64<CHK, GS>(O, N, queue, qn, nr_grp, G, acc, cnt);
+  if (qn) drain64<CHK ? DR_FLAG : DR_NOCHK, GS>(O, N, queue, qn, nr_grp, G, acc, cnt);
   __syncthreads();
   grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
 }
@@ -537,7 +438,7 @@ static mb_status fw_gs(int gs, const DevPrg &P, const mb_op &O, uint32_t nr_grp,
   }
 }
 
-int shape_of(const mb_op &O, uint32_t nr_grp, uint32_t sure, ShapeArgs *A, bool *narrow) {
+int shape_of(const mb_op &O, uint32_t nr_grp, uint32_t sure, ShapeArgs *A, bool *narrow, uint32_t keyed) {
   memset(A, 0, sizeof(*A));
   A->ng = nr_grp;
   if (O.nsrc > 6) return -1;
@@ -570,9 +471,9 @@ int shape_of(const mb_op &O, uint32_t nr_grp, uint32_t sure, ShapeArgs *A, bool 
       continue;
     for (int nar = 0; nar < 2; ++nar) {
       bool same = true;
-      for (uint32_t s = 0; s < b.ns && same; ++s) same = !O.src[s].fk && O.src[s].width == SHAPE_W[i][nar][s];
+      for (uint32_t s = 0; s < b.ns && same; ++s) same = (!O.src[s].fk || (keyed >> s & 1u)) && O.src[s].width == SHAPE_W[i][nar][s];
       if (!same) continue;
-      for (uint32_t s = 0; s < b.ns; ++s) A->col[s] = O.src[s].col;
+      for (uint32_t s = 0; s < b.ns; ++s) A->col[s] = O.src[s].col, A->fk[s] = O.src[s].fk;
       *narrow = nar != 0;
       return (int)i;
     }

@@ -1,9 +1,9 @@
 // grpby.cu - the query kernels: fused program -> compaction -> op -> group-by
-// (mb_vprg_grpby), the no-index scan (mb_join_grpby) and the three
-// materialised stages (mb_vprg_eval, mb_bitmap_to_rows, mb_rows_grpby).
+// (mb_vprg_grpby) and the three materialised stages (mb_vprg_eval,
+// mb_bitmap_to_rows, mb_rows_grpby).
 //
-// Reference kernels: vprg_grpby (primitive.cuh:340-445), grpby
-// (primitive.cuh:16-48), abla::_stg1/_stg2/_stg3 (primitive_abla.cuh:262-394).
+// Reference kernels: vprg_grpby (primitive.cuh:340-445),
+// abla::_stg1/_stg2/_stg3 (primitive_abla.cuh:262-394).
 //
 // B200 design of the fused kernel:
 //  - Persistent grid (SMs x occupancy).  Work unit = one warp tile of 32*V
@@ -139,7 +139,7 @@ void detect_cnf(DevPrg *o) {
   o->neg = neg;
 }
 
-static mb_status validate_op(const mb_op *op) {
+mb_status validate_op(const mb_op *op) {
   if (!op) return fail(MB_ERR_INVALID, "op is NULL");
   if (op->nsrc > MB_MAXSRC) return fail(MB_ERR_INVALID, "op: %u sources > %d", op->nsrc, MB_MAXSRC);
   for (uint32_t i = 0; i < op->nsrc; ++i) {
@@ -235,127 +235,6 @@ vbp_grpby_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ mb_op
       aggregate<GS>(G, kept, grp, val, acc);
     }
     __syncwarp();
-  }
-  __syncthreads();
-  grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
-}
-
-// -------------------------------------------------------- no-index scan
-// Clause c alone on one row, as op_eval evaluates it.
-__device__ __forceinline__ bool clause_pass(const mb_op &O, uint32_t c, uint32_t t0, uint32_t row) {
-  bool any = false;
-  for (uint32_t k = 0; k < O.clause_len[c] && !any; ++k) {
-    const mb_term &tm = O.terms[t0 + k];
-    uint64_t v;
-    any = src_value(O.src[tm.src], row, v) && v >= tm.lo && v < tm.hi;
-  }
-  return any;
-}
-
-constexpr uint32_t JQ = 160;  // rows a warp queues between the screen and the op (31 + a 128-row chunk)
-
-// Every row through the op.  A row first meets one clause (`screen`, first
-// term `t0`; none if screen >= nclause), one row per lane; the rows that pass
-// queue per warp, and each full warp of them runs the rest of the op, so the
-// lanes of its loads and branches are all live rows.  The result equals
-// op_eval on every row (the screen is one of the op's own clauses).
-// Four consecutive values of a fact column of SW-byte elements from one
-// vector load (the column 16-byte aligned, rows r .. r+3 inside it, r a
-// multiple of 4).
-template <int SW>
-__device__ __forceinline__ void load4(const void *col, uint64_t r, uint64_t (&v)[4]) {
-  if (SW == 1) {
-    const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(col) + r / 4);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = (w >> (8 * j)) & 0xffu;
-  } else if (SW == 2) {
-    const uint2 w = __ldg(reinterpret_cast<const uint2 *>(col) + r / 4);
-    v[0] = w.x & 0xffffu, v[1] = w.x >> 16, v[2] = w.y & 0xffffu, v[3] = w.y >> 16;
-  } else if (SW == 4) {
-    const uint4 w = __ldg(reinterpret_cast<const uint4 *>(col) + r / 4);
-    v[0] = w.x, v[1] = w.y, v[2] = w.z, v[3] = w.w;
-  } else {
-    const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(col) + r / 2),
-                     b = __ldg(reinterpret_cast<const ulonglong2 *>(col) + r / 2 + 1);
-    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
-  }
-}
-
-template <int GS, int SW>
-__global__ void __launch_bounds__(256, 8)
-join_grpby_kernel(uint64_t nrows, const __grid_constant__ mb_op O, uint32_t nr_grp, uint32_t hcap,
-                  uint32_t grp_bytes, uint32_t screen, uint32_t t0, unsigned long long *__restrict__ out,
-                  unsigned long long *__restrict__ nqual) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ uint64_t red[64];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  GrpCtx G = grp_init<GS>(smem, nr_grp, hcap, out);
-  uint32_t *queue = reinterpret_cast<uint32_t *>(smem + grp_bytes) + (size_t)warp * JQ;
-  __syncthreads();
-  int64_t acc = 0;
-  uint64_t cnt = 0;
-  uint32_t qn = 0;
-  const uint32_t lt = (1u << lane) - 1u;
-  auto drain = [&](uint32_t m) {  // the last m (<= 32) queued rows through the op
-    bool kept = false;
-    int64_t val = 0;
-    uint32_t grp = 0;
-    if (lane < m) kept = op_eval(O, queue[qn - m + lane], true, nr_grp, val, grp, screen);
-    cnt += kept ? 1u : 0u;
-    aggregate<GS>(G, kept, grp, val, acc);
-    qn -= m;
-    __syncwarp();
-  };
-  const uint64_t nchunks = (nrows + 31) / 32;
-  if (screen >= O.nclause) {  // no screen (or no room for the queues): every row through the op
-    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nchunks; ch += (uint64_t)gridDim.x * nw) {
-      const uint64_t row = ch * 32 + lane;
-      bool kept = false;
-      int64_t val = 0;
-      uint32_t grp = 0;
-      if (row < nrows) kept = op_eval(O, (uint32_t)row, true, nr_grp, val, grp);
-      cnt += kept ? 1u : 0u;
-      aggregate<GS>(G, kept, grp, val, acc);
-    }
-  } else if (SW == 0) {
-    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nchunks; ch += (uint64_t)gridDim.x * nw) {
-      const uint64_t row = ch * 32 + lane;
-      const bool pass = row < nrows && clause_pass(O, screen, t0, (uint32_t)row);
-      const uint32_t bal = __ballot_sync(0xffffffffu, pass);
-      if (pass) queue[qn + __popc(bal & lt)] = (uint32_t)row;
-      qn += __popc(bal);  // at most 31 + 32 < JQ
-      __syncwarp();
-      if (qn >= 32) drain(32);
-    }
-    if (qn) drain(qn);
-  } else {
-    // the screen is one range on a fact column of SW-byte elements: four rows
-    // a lane from one vector load; 128-row chunks, the last one partly by
-    // scalar loads
-    const mb_term &tm = O.terms[t0];
-    const void *col = O.src[tm.src].col;
-    const uint64_t lo = tm.lo, hi = tm.hi, nch4 = (nrows + 127) / 128;
-    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nch4; ch += (uint64_t)gridDim.x * nw) {
-      const uint64_t r = ch * 128 + 4 * lane;
-      uint64_t v[4] = {0, 0, 0, 0};
-      if (ch * 128 + 128 <= nrows) {
-        load4<SW>(col, r, v);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (r + j < nrows) v[j] = load_width(col, r + j, SW);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool pass = r + j < nrows && v[j] >= lo && v[j] < hi;
-        const uint32_t bal = __ballot_sync(0xffffffffu, pass);
-        if (pass) queue[qn + __popc(bal & lt)] = (uint32_t)(r + j);
-        qn += __popc(bal);  // at most 31 + 128 < JQ
-      }
-      __syncwarp();
-      while (qn >= 32) drain(32);
-    }
-    if (qn) drain(qn);
   }
   __syncthreads();
   grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
@@ -531,7 +410,7 @@ mb_status certain_of(uint32_t *p, const uint32_t *u, uint64_t nrows, cudaStream_
 constexpr uint32_t DEFAULT_HCAP = 4096;
 constexpr uint32_t SHARED_MAX_GROUPS = 8192;
 
-static int pick_gs(uint32_t nr_grp, uint32_t requested) {
+int pick_gs(uint32_t nr_grp, uint32_t requested) {
   if (nr_grp == 1 && requested != MB_GRP_GLOBAL && requested != MB_GRP_HASH) return GS_SCALAR;
   switch (requested) {
   case MB_GRP_SHARED: return GS_SHARED;
@@ -639,91 +518,6 @@ mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_
 extern "C" mb_status mb_vprg_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_t *out,
                                    uint64_t *nqual, const mb_launch *launch, void *stream) {
   return fused_grpby(p, op, nr_grp, out, nqual, launch, as_stream(stream), true, 0);
-}
-
-// The clause that screens rows in the no-index scan: the first whose terms
-// read fact columns only (one load a row), else the first; nclause if none.
-static uint32_t screen_clause(const mb_op &O, uint32_t *t0) {
-  uint32_t t = 0, first_t = 0;
-  for (uint32_t c = 0; c < O.nclause; ++c) {
-    bool fact = true;
-    for (uint32_t k = 0; k < O.clause_len[c]; ++k)
-      if (O.src[O.terms[t + k].src].fk) fact = false;
-    if (fact) {
-      *t0 = t;
-      return c;
-    }
-    t += O.clause_len[c];
-  }
-  *t0 = first_t;
-  return 0;
-}
-
-template <int GS, int SW>
-static mb_status launch_join_sw(uint64_t n, const mb_op &O, uint32_t nr_grp, uint32_t hcap, int64_t *out,
-                                uint64_t *nqual, cudaStream_t st, uint32_t screen, uint32_t t0) {
-  auto kern = join_grpby_kernel<GS, SW>;
-  const uint32_t warps = 8;
-  const size_t gb = (grp_smem_bytes(GS, nr_grp, hcap) + 15) & ~(size_t)15;
-  // the row queues only where they cost no resident CTA (a large group
-  // table in shared memory can leave no room for them)
-  const size_t qbytes = (size_t)warps * JQ * 4;
-  if (screen < O.nclause) {
-    const size_t cap = (size_t)dev_info().max_smem_optin - 1024;  // room for the kernel's static shared memory
-    int with = 0, without = 0;
-    MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min(cap, gb + qbytes)));
-    if (gb + qbytes <= cap)
-      MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&with, kern, (int)(warps * 32), gb + qbytes));
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&without, kern, (int)(warps * 32), gb));
-    if (with < without) screen = O.nclause;
-  }
-  const size_t smem = gb + (screen < O.nclause ? qbytes : 0);
-  LaunchShape ls;
-  MB_CHECK(shape_for(kern, warps, smem, (n + 31) / 32, &ls, 0));
-  kern<<<ls.grid, ls.block, ls.smem, st>>>(n, O, nr_grp, hcap, (uint32_t)gb, screen, t0,
-                                           reinterpret_cast<unsigned long long *>(out),
-                                           reinterpret_cast<unsigned long long *>(nqual));
-  MB_LAUNCH_CHECK("join_grpby_kernel");
-  return MB_OK;
-}
-
-// The screen's shape picks the kernel: one range on a 16-byte-aligned fact
-// column screens four rows a lane (its width a template argument).
-template <int GS>
-static mb_status launch_join(uint64_t n, const mb_op &O, uint32_t nr_grp, uint32_t hcap, int64_t *out,
-                             uint64_t *nqual, cudaStream_t st) {
-  uint32_t t0 = 0;
-  const uint32_t screen = screen_clause(O, &t0);
-  uint32_t sw = 0;
-  if (screen < O.nclause && O.clause_len[screen] == 1) {
-    const mb_src &s = O.src[O.terms[t0].src];
-    if (!s.fk && (reinterpret_cast<uintptr_t>(s.col) & 15) == 0) sw = s.width;
-  }
-  switch (sw) {
-  case 1: return launch_join_sw<GS, 1>(n, O, nr_grp, hcap, out, nqual, st, screen, t0);
-  case 2: return launch_join_sw<GS, 2>(n, O, nr_grp, hcap, out, nqual, st, screen, t0);
-  case 4: return launch_join_sw<GS, 4>(n, O, nr_grp, hcap, out, nqual, st, screen, t0);
-  case 8: return launch_join_sw<GS, 8>(n, O, nr_grp, hcap, out, nqual, st, screen, t0);
-  default: return launch_join_sw<GS, 0>(n, O, nr_grp, hcap, out, nqual, st, screen, t0);
-  }
-}
-
-extern "C" mb_status mb_join_grpby(uint64_t nrows, const mb_op *op, uint32_t nr_grp, int64_t *out,
-                                   uint64_t *nqual, void *stream) {
-  if (!out || !nqual) return fail(MB_ERR_INVALID, "mb_join_grpby: NULL output");
-  if (nr_grp == 0) return fail(MB_ERR_INVALID, "mb_join_grpby: nr_grp == 0");
-  MB_CHECK(validate_op(op));
-  if (nrows >= (1ull << 32)) return fail(MB_ERR_INVALID, "mb_join_grpby: rows >= 2^32");
-  cudaStream_t st = as_stream(stream);
-  MB_CUDA(cudaMemsetAsync(out, 0, (size_t)nr_grp * sizeof(int64_t), st));
-  MB_CUDA(cudaMemsetAsync(nqual, 0, sizeof(uint64_t), st));
-  if (nrows == 0) return MB_OK;
-  const int gs = pick_gs(nr_grp, MB_GRP_AUTO);
-  switch (gs) {
-  case GS_SCALAR: return launch_join<GS_SCALAR>(nrows, *op, nr_grp, DEFAULT_HCAP, out, nqual, st);
-  case GS_SHARED: return launch_join<GS_SHARED>(nrows, *op, nr_grp, DEFAULT_HCAP, out, nqual, st);
-  default: return launch_join<GS_GLOBAL>(nrows, *op, nr_grp, DEFAULT_HCAP, out, nqual, st);
-  }
 }
 
 extern "C" mb_status mb_vprg_eval(const mb_vprg *p, int chk, uint32_t *possible, uint32_t *uncertain,
@@ -879,414 +673,4 @@ extern "C" mb_status mb_bitmap_to_rows_noalloc(const uint32_t *possible, const u
   rows_write_kernel<<<(unsigned)nseg, RL_THREADS, 0, st>>>(possible, uncertain, nrows, seg, rows);
   MB_LAUNCH_CHECK("rows_write_kernel");
   return MB_OK;
-}
-
-// ------------------------------------------------------- hash-join plan
-// Crystal-style join plan (the reference's comparison system, crystal/src/ssb/q21.cu and
-// its siblings: build a hash table per filtered dimension, then one pass over the fact rows
-// probes them).  For every foreign key whose dimension attributes carry a predicate of their
-// own (a clause all of whose terms read that dimension), the dimension rows passing those
-// clauses go into an open-addressing table keyed by dimension key and carrying the
-// attributes the op reads; the probe pass evaluates the fact-column clauses first, then looks
-// each key up (a miss eliminates the row), then the remaining clauses, group key and value.
-// Tables up to HJ_SMEM_MAX bytes are copied into every CTA's shared memory.  Results equal
-// mb_join_grpby's on the same op.
-namespace mb {
-
-constexpr uint32_t HJ_MAXT = 4;                 // tables (distinct foreign keys) per op
-constexpr uint32_t HJ_PAY = 3;                  // attributes one entry carries
-constexpr uint32_t HJ_SMEM_MAX = 48 * 1024;     // per staged table
-constexpr uint32_t HJ_SMEM_TOTAL = 128 * 1024;  // all staged tables
-
-struct HjTable {
-  const uint32_t *fk;
-  uint64_t dimsz;
-  uint4 *slots;       // {key, a0, a1, a2}; key HASH_EMPTY = free
-  uint32_t mask;      // capacity - 1
-  uint32_t npay;
-  uint32_t pushed;    // clauses evaluated at the build
-  uint32_t smem_off;  // byte offset of the staged copy, or ~0u
-  uint32_t pay_src[HJ_PAY];
-};
-
-struct HjPlan {
-  uint32_t ntab;
-  HjTable tab[HJ_MAXT];
-  int32_t src_tab[MB_MAXSRC];   // table carrying source s, -1: read directly
-  uint32_t src_pay[MB_MAXSRC];  // its slot in the entry
-  uint32_t fact_clauses;        // probe clauses that read fact columns only
-  uint32_t late_clauses;        // the other probe clauses
-  uint32_t term0[MB_MAXCLAUSE]; // first term of each clause
-  uint32_t smem_tables;         // bytes of the staged tables (the row queues follow)
-};
-
-// Clauses `mask` on dimension row d of table t (sources read at index d).
-__device__ __forceinline__ bool hj_dim_pass(const mb_op &O, const HjPlan &H, uint32_t mask, uint64_t d) {
-  for (uint32_t c = 0; c < O.nclause; ++c) {
-    if (!(mask >> c & 1u)) continue;
-    bool any = false;
-    for (uint32_t k = 0, t = H.term0[c]; k < O.clause_len[c] && !any; ++k, ++t) {
-      const mb_term &tm = O.terms[t];
-      const uint64_t v = load_width(O.src[tm.src].col, d, O.src[tm.src].width);
-      any = v >= tm.lo && v < tm.hi;
-    }
-    if (!any) return false;
-  }
-  return true;
-}
-
-__global__ void hj_count_kernel(const __grid_constant__ mb_op O, const __grid_constant__ HjPlan H, uint32_t t,
-                                unsigned long long *count) {
-  const HjTable &T = H.tab[t];
-  uint32_t c = 0;
-  for (uint64_t d = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; d < T.dimsz; d += (uint64_t)gridDim.x * blockDim.x)
-    c += hj_dim_pass(O, H, T.pushed, d) ? 1u : 0u;
-  for (int o = 16; o; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count + t, (unsigned long long)c);
-}
-
-// Inserts the passing dimension rows of table t.  The walk from a key's hash
-// slot ends within the table: it holds at most half as many rows as slots.
-__global__ void hj_insert_kernel(const __grid_constant__ mb_op O, const __grid_constant__ HjPlan H, uint32_t t) {
-  const HjTable &T = H.tab[t];
-  for (uint64_t d = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; d < T.dimsz;
-       d += (uint64_t)gridDim.x * blockDim.x) {
-    if (!hj_dim_pass(O, H, T.pushed, d)) continue;
-    uint32_t a[HJ_PAY] = {0, 0, 0};
-    for (uint32_t j = 0; j < T.npay; ++j) {
-      const mb_src &s = O.src[T.pay_src[j]];
-      a[j] = (uint32_t)load_width(s.col, d, s.width);
-    }
-    uint32_t h = hash32((uint32_t)d) & T.mask;
-    for (uint32_t p = 0; p <= T.mask; ++p, h = (h + 1) & T.mask)
-      if (atomicCAS(&T.slots[h].x, HASH_EMPTY, (uint32_t)d) == HASH_EMPTY) {
-        T.slots[h].y = a[0], T.slots[h].z = a[1], T.slots[h].w = a[2];
-        break;
-      }
-  }
-}
-
-// Value of source s at `row`: a table's attribute, or a direct read (as
-// src_value: false when a foreign key is out of its dimension).
-__device__ __forceinline__ bool hj_value(const mb_op &O, const HjPlan &H, uint32_t s, uint32_t row,
-                                         const uint32_t *got, uint64_t &v) {
-  const int32_t t = H.src_tab[s];
-  if (t >= 0) {
-    v = got[t * HJ_PAY + H.src_pay[s]];
-    return true;
-  }
-  return src_value(O.src[s], row, v);
-}
-
-__device__ __forceinline__ bool hj_clauses(const mb_op &O, const HjPlan &H, uint32_t mask, uint32_t row,
-                                           const uint32_t *got) {
-  for (uint32_t c = 0; c < O.nclause; ++c) {
-    if (!(mask >> c & 1u)) continue;
-    bool any = false;
-    for (uint32_t k = 0, t = H.term0[c]; k < O.clause_len[c] && !any; ++k, ++t) {
-      const mb_term &tm = O.terms[t];
-      uint64_t v;
-      any = hj_value(O, H, tm.src, row, got, v) && v >= tm.lo && v < tm.hi;
-    }
-    if (!any) return false;
-  }
-  return true;
-}
-
-// The op on a row whose fact-column clauses already passed.
-__device__ __forceinline__ bool hj_row(const mb_op &O, const HjPlan &H, const uint4 *const *tabs, uint32_t row,
-                                       uint32_t nr_grp, int64_t &value, uint32_t &group) {
-  uint32_t got[HJ_MAXT * HJ_PAY];
-  for (uint32_t t = 0; t < H.ntab; ++t) {
-    const HjTable &T = H.tab[t];
-    const uint32_t key = __ldg(T.fk + row);
-    uint32_t h = hash32(key) & T.mask;
-    const uint4 *tab = tabs[t];
-    for (;;) {  // at least half the slots are free: the walk ends
-      const uint4 e = tab[h];
-      if (e.x == key) {
-        got[t * HJ_PAY + 0] = e.y, got[t * HJ_PAY + 1] = e.z, got[t * HJ_PAY + 2] = e.w;
-        break;
-      }
-      if (e.x == HASH_EMPTY) return false;
-      h = (h + 1) & T.mask;
-    }
-  }
-  if (!hj_clauses(O, H, H.late_clauses, row, got)) return false;
-  uint32_t g = 0;
-  for (uint32_t k = 0; k < O.nkey; ++k) {
-    const mb_key &kk = O.keys[k];
-    uint64_t v;
-    if (!hj_value(O, H, kk.src, row, got, v)) return false;
-    uint32_t x = (uint32_t)v;
-    if (kk.xform == MB_X_DIV) x = (uint32_t)(v / kk.div);
-    else if (kk.xform == MB_X_YEAR) x = date_to_year((uint32_t)v);
-    g += kk.mul * (x - kk.base);
-  }
-  if (g >= nr_grp) return false;
-  uint64_t a = 0, b = 0;
-  switch (O.vkind) {
-  case MB_V_ONE: value = 1; break;
-  case MB_V_COL:
-    if (!hj_value(O, H, O.va, row, got, a)) return false;
-    value = (int64_t)a;
-    break;
-  case MB_V_MUL:
-    if (!hj_value(O, H, O.va, row, got, a) || !hj_value(O, H, O.vb, row, got, b)) return false;
-    value = (int64_t)(a * b);
-    break;
-  default:
-    if (!hj_value(O, H, O.va, row, got, a) || !hj_value(O, H, O.vb, row, got, b)) return false;
-    value = (int64_t)a - (int64_t)b;
-    break;
-  }
-  group = g;
-  return true;
-}
-
-template <int GS, int SW>
-__global__ void __launch_bounds__(SW ? 256 : 512, SW ? 4 : 1)
-hj_probe_kernel(uint64_t nrows, const __grid_constant__ mb_op O, const __grid_constant__ HjPlan H, uint32_t nr_grp,
-                uint32_t hcap, uint32_t grp_bytes, uint32_t t0, unsigned long long *__restrict__ out,
-                unsigned long long *__restrict__ nqual) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ uint64_t red[64];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  GrpCtx G = grp_init<GS>(smem, nr_grp, hcap, out);
-  const uint4 *tabs[HJ_MAXT];
-  for (uint32_t t = 0; t < HJ_MAXT; ++t) {
-    tabs[t] = nullptr;
-    if (t >= H.ntab) continue;
-    const HjTable &T = H.tab[t];
-    if (T.smem_off == ~0u) {
-      tabs[t] = T.slots;
-      continue;
-    }
-    uint4 *dst = reinterpret_cast<uint4 *>(smem + grp_bytes + T.smem_off);
-    for (uint32_t i = threadIdx.x; i <= T.mask; i += blockDim.x) dst[i] = T.slots[i];
-    tabs[t] = dst;
-  }
-  __syncthreads();
-  int64_t acc = 0;
-  uint64_t cnt = 0;
-  // as the no-index scan: the fact-column clauses screen the rows one per
-  // lane, the rows that pass queue per warp and full warps of them probe
-  uint32_t *queue = reinterpret_cast<uint32_t *>(smem + grp_bytes + H.smem_tables) + (size_t)warp * JQ;
-  uint32_t qn = 0;
-  const uint32_t lt = (1u << lane) - 1u;
-  auto drain = [&](uint32_t m) {
-    bool kept = false;
-    int64_t val = 0;
-    uint32_t grp = 0;
-    if (lane < m) kept = hj_row(O, H, tabs, queue[qn - m + lane], nr_grp, val, grp);
-    cnt += kept ? 1u : 0u;
-    aggregate<GS>(G, kept, grp, val, acc);
-    qn -= m;
-    __syncwarp();
-  };
-  if (SW == 0) {
-    const uint64_t nchunks = (nrows + 31) / 32;
-    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nchunks; ch += (uint64_t)gridDim.x * nw) {
-      const uint64_t row = ch * 32 + lane;
-      const bool pass = row < nrows && hj_clauses(O, H, H.fact_clauses, (uint32_t)row, nullptr);
-      const uint32_t bal = __ballot_sync(0xffffffffu, pass);
-      if (pass) queue[qn + __popc(bal & lt)] = (uint32_t)row;
-      qn += __popc(bal);
-      __syncwarp();
-      if (qn >= 32) drain(32);
-    }
-  } else {
-    // the fact clauses are one range on an aligned column: four rows a lane
-    // from one vector load, as the no-index scan screens
-    const mb_term &tm = O.terms[t0];
-    const void *col = O.src[tm.src].col;
-    const uint64_t lo = tm.lo, hi = tm.hi, nch4 = (nrows + 127) / 128;
-    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nch4; ch += (uint64_t)gridDim.x * nw) {
-      const uint64_t r = ch * 128 + 4 * lane;
-      uint64_t v[4] = {0, 0, 0, 0};
-      if (ch * 128 + 128 <= nrows) {
-        load4<SW>(col, r, v);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (r + j < nrows) v[j] = load_width(col, r + j, SW);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool pass = r + j < nrows && v[j] >= lo && v[j] < hi;
-        const uint32_t bal = __ballot_sync(0xffffffffu, pass);
-        if (pass) queue[qn + __popc(bal & lt)] = (uint32_t)(r + j);
-        qn += __popc(bal);  // at most 31 + 128 < JQ
-      }
-      __syncwarp();
-      while (qn >= 32) drain(32);
-    }
-  }
-  if (qn) drain(qn);
-  __syncthreads();
-  grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
-}
-
-template <int GS, int SW>
-static mb_status launch_hj_sw(uint64_t n, const mb_op &O, const HjPlan &H, uint32_t smem_tables, uint32_t nr_grp,
-                              int64_t *out, uint64_t *nqual, cudaStream_t st, uint32_t t0);
-
-// The probe's screen shape picks the kernel: the fact clauses one range on a
-// 16-byte-aligned fact column screen four rows a lane.
-template <int GS>
-static mb_status launch_hj(uint64_t n, const mb_op &O, const HjPlan &H, uint32_t smem_tables, uint32_t nr_grp,
-                           int64_t *out, uint64_t *nqual, cudaStream_t st) {
-  uint32_t sw = 0, t0 = 0;
-  const uint32_t fc = H.fact_clauses;
-  if (fc && !(fc & (fc - 1))) {
-    const uint32_t c = (uint32_t)__builtin_ctz(fc);
-    if (O.clause_len[c] == 1) {
-      t0 = H.term0[c];
-      const mb_src &s = O.src[O.terms[t0].src];
-      if (!s.fk && (reinterpret_cast<uintptr_t>(s.col) & 15) == 0) sw = s.width;
-    }
-  }
-  switch (sw) {
-  case 1: return launch_hj_sw<GS, 1>(n, O, H, smem_tables, nr_grp, out, nqual, st, t0);
-  case 2: return launch_hj_sw<GS, 2>(n, O, H, smem_tables, nr_grp, out, nqual, st, t0);
-  case 4: return launch_hj_sw<GS, 4>(n, O, H, smem_tables, nr_grp, out, nqual, st, t0);
-  case 8: return launch_hj_sw<GS, 8>(n, O, H, smem_tables, nr_grp, out, nqual, st, t0);
-  default: return launch_hj_sw<GS, 0>(n, O, H, smem_tables, nr_grp, out, nqual, st, t0);
-  }
-}
-
-template <int GS, int SW>
-static mb_status launch_hj_sw(uint64_t n, const mb_op &O, const HjPlan &H, uint32_t smem_tables, uint32_t nr_grp,
-                              int64_t *out, uint64_t *nqual, cudaStream_t st, uint32_t t0) {
-  auto kern = hj_probe_kernel<GS, SW>;
-  const uint32_t warps = 8;
-  const size_t grp_bytes = (grp_smem_bytes(GS, nr_grp, DEFAULT_HCAP) + 15) & ~(size_t)15;
-  LaunchShape ls;
-  MB_CHECK(shape_for(kern, warps, grp_bytes + smem_tables + (size_t)warps * JQ * 4, (n + 31) / 32, &ls, 0));
-  kern<<<ls.grid, ls.block, ls.smem, st>>>(n, O, H, nr_grp, DEFAULT_HCAP, (uint32_t)grp_bytes, t0,
-                                           reinterpret_cast<unsigned long long *>(out),
-                                           reinterpret_cast<unsigned long long *>(nqual));
-  MB_LAUNCH_CHECK("hj_probe_kernel");
-  return MB_OK;
-}
-
-}  // namespace mb
-
-extern "C" mb_status mb_hash_join_grpby(uint64_t nrows, const mb_op *op, uint32_t nr_grp, int64_t *out,
-                                        uint64_t *nqual, void *stream) {
-  using namespace mb;
-  if (!out || !nqual) return fail(MB_ERR_INVALID, "mb_hash_join_grpby: NULL output");
-  if (nr_grp == 0) return fail(MB_ERR_INVALID, "mb_hash_join_grpby: nr_grp == 0");
-  MB_CHECK(validate_op(op));
-  if (nrows >= (1ull << 32)) return fail(MB_ERR_INVALID, "mb_hash_join_grpby: rows >= 2^32");
-  const mb_op &O = *op;
-  HjPlan H;
-  memset(&H, 0, sizeof(H));
-  for (uint32_t s = 0; s < MB_MAXSRC; ++s) H.src_tab[s] = -1;
-  uint32_t t0 = 0;
-  for (uint32_t c = 0; c < O.nclause; ++c) H.term0[c] = t0, t0 += O.clause_len[c];
-  // clauses whose terms all read one foreign key's dimension go into that key's table
-  uint32_t pushed_any = 0;
-  for (uint32_t c = 0; c < O.nclause; ++c) {
-    const uint32_t *fk = nullptr;
-    bool one = O.clause_len[c] > 0;
-    for (uint32_t k = 0; k < O.clause_len[c]; ++k) {
-      const mb_src &s = O.src[O.terms[H.term0[c] + k].src];
-      if (!s.fk || s.dimsz == 0 || s.width > 4 || (fk && s.fk != fk)) one = false;
-      fk = s.fk;
-    }
-    if (!one) continue;
-    uint32_t t = 0;
-    while (t < H.ntab && H.tab[t].fk != fk) ++t;
-    if (t == H.ntab) {
-      if (H.ntab == HJ_MAXT) continue;  // more keys than tables: probe this clause directly
-      H.tab[t].fk = fk;
-      H.tab[t].dimsz = ~0ull;
-      ++H.ntab;
-    }
-    H.tab[t].pushed |= 1u << c;
-    pushed_any |= 1u << c;
-  }
-  // each table carries every source on its key (the op may read them later)
-  for (uint32_t t = 0; t < H.ntab; ++t) {
-    HjTable &T = H.tab[t];
-    for (uint32_t s = 0; s < O.nsrc; ++s) {
-      if (O.src[s].fk != T.fk) continue;
-      if (O.src[s].width > 4 || T.npay == HJ_PAY)
-        return fail(MB_ERR_UNSUPPORTED, "mb_hash_join_grpby: more than %u attributes (or one over 4 bytes) on one key",
-                    HJ_PAY);
-      T.dimsz = std::min<uint64_t>(T.dimsz, O.src[s].dimsz ? O.src[s].dimsz : ~0ull);
-      H.src_tab[s] = (int32_t)t;
-      H.src_pay[s] = T.npay;
-      T.pay_src[T.npay++] = s;
-    }
-  }
-  for (uint32_t c = 0; c < O.nclause; ++c) {
-    if (pushed_any >> c & 1u) continue;
-    bool fact = true;
-    for (uint32_t k = 0; k < O.clause_len[c]; ++k)
-      if (O.src[O.terms[H.term0[c] + k].src].fk) fact = false;
-    (fact ? H.fact_clauses : H.late_clauses) |= 1u << c;
-  }
-  cudaStream_t st = as_stream(stream);
-  MB_CUDA(cudaMemsetAsync(out, 0, (size_t)nr_grp * sizeof(int64_t), st));
-  MB_CUDA(cudaMemsetAsync(nqual, 0, sizeof(uint64_t), st));
-  if (nrows == 0) return MB_OK;
-  // build: count the passing dimension rows of every table (one wait), size
-  // each table to a power of two >= 2 x its rows, insert
-  uint64_t cnt[HJ_MAXT] = {0, 0, 0, 0};
-  if (H.ntab) {
-    Scratch sc(st);  // freed after the probe, in stream order
-    unsigned long long *dcnt;
-    MB_CHECK(sc.get(&dcnt, HJ_MAXT));
-    MB_CUDA(cudaMemsetAsync(dcnt, 0, 8 * HJ_MAXT, st));
-    for (uint32_t t = 0; t < H.ntab; ++t) {
-      const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(H.tab[t].dimsz, 256), (uint64_t)dev_info().sms * 8);
-      hj_count_kernel<<<grid, 256, 0, st>>>(O, H, t, dcnt);
-      MB_LAUNCH_CHECK("hj_count_kernel");
-    }
-    MB_CUDA(cudaMemcpyAsync(cnt, dcnt, 8 * HJ_MAXT, cudaMemcpyDeviceToHost, st));
-    MB_CUDA(cudaStreamSynchronize(st));
-    for (uint32_t t = 0; t < H.ntab; ++t)
-      if (cnt[t] == 0) return MB_OK;  // a dimension with no passing row: nothing qualifies
-    uint64_t off = 0, smem_tables = 0;
-    uint64_t offs[HJ_MAXT];
-    for (uint32_t t = 0; t < H.ntab; ++t) {
-      if (cnt[t] > (1ull << 30))
-        return fail(MB_ERR_UNSUPPORTED, "mb_hash_join_grpby: %llu dimension rows in one table (at most 2^30)",
-                    (unsigned long long)cnt[t]);
-      uint64_t capt = 64;
-      while (capt < 2 * cnt[t]) capt <<= 1;
-      H.tab[t].mask = (uint32_t)(capt - 1);
-      offs[t] = off;
-      off += capt * 16;
-      H.tab[t].smem_off = ~0u;
-      if (capt * 16 <= HJ_SMEM_MAX && smem_tables + capt * 16 <= HJ_SMEM_TOTAL) {
-        H.tab[t].smem_off = (uint32_t)smem_tables;
-        smem_tables += capt * 16;
-      }
-    }
-    uint8_t *base;
-    MB_CHECK(sc.get(&base, off));
-    for (uint32_t t = 0; t < H.ntab; ++t) {
-      H.tab[t].slots = reinterpret_cast<uint4 *>(base + offs[t]);
-      MB_CUDA(cudaMemsetAsync(H.tab[t].slots, 0xff, (size_t)(H.tab[t].mask + 1) * 16, st));
-    }
-    for (uint32_t t = 0; t < H.ntab; ++t) {
-      const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(H.tab[t].dimsz, 256), (uint64_t)dev_info().sms * 8);
-      hj_insert_kernel<<<grid, 256, 0, st>>>(O, H, t);
-      MB_LAUNCH_CHECK("hj_insert_kernel");
-    }
-    H.smem_tables = (uint32_t)smem_tables;
-    const int gs = pick_gs(nr_grp, MB_GRP_AUTO);
-    mb_status r;
-    switch (gs) {
-    case GS_SCALAR: r = launch_hj<GS_SCALAR>(nrows, O, H, (uint32_t)smem_tables, nr_grp, out, nqual, st); break;
-    case GS_SHARED: r = launch_hj<GS_SHARED>(nrows, O, H, (uint32_t)smem_tables, nr_grp, out, nqual, st); break;
-    default: r = launch_hj<GS_GLOBAL>(nrows, O, H, (uint32_t)smem_tables, nr_grp, out, nqual, st); break;
-    }
-    return r;
-  }
-  // no table to build: the plain scan
-  return mb_join_grpby(nrows, op, nr_grp, out, nqual, stream);
 }

@@ -33,6 +33,7 @@ struct ShapeKey {
 
 struct ShapeArgs {
   const void *col[6];
+  const uint32_t *fk[6];  // the row's index into col, or NULL: the row itself (kernels with JOIN)
   uint32_t lo[6], hi[6];  // candidate-check bounds, inclusive
   ShapeKey key[4];        // by slot (key slots are 0..3)
   uint32_t ng;
@@ -40,11 +41,13 @@ struct ShapeArgs {
 };
 
 // Host: the shape of an op (BSHAPES index, -1: none) with its arguments;
-// *narrow selects the SHAPE_W row.  Sources through a foreign key, widths of
+// *narrow selects the SHAPE_W row.  Sources through a foreign key (but `keyed`), widths of
 // neither layout, clauses of several terms, ranges no value meets and keys
 // sharing a source have no shape.
 // sure: clauses (bit c) that every candidate row is known to satisfy.
-int shape_of(const mb_op &O, uint32_t nr_grp, uint32_t sure, ShapeArgs *A, bool *narrow);
+// keyed: sources (bit s) whose foreign key lies inside its dimension on every
+// candidate row; only those may be read through one.
+int shape_of(const mb_op &O, uint32_t nr_grp, uint32_t sure, ShapeArgs *A, bool *narrow, uint32_t keyed = 0);
 
 template <int W>
 __device__ __forceinline__ uint32_t shape_load(const void *col, uint32_t row) {
@@ -64,8 +67,8 @@ struct ShapeSlot {
   static constexpr int w = SHAPE_W[SH][NARROW ? 1 : 0][S];
 };
 
-// One row's slots, 0..5.
-template <int SH, bool NARROW>
+// One row's slots, 0..5.  JOIN: slots may be read through a foreign key.
+template <int SH, bool NARROW, bool JOIN>
 struct ShapeVals {
   static constexpr BShape sh = BSHAPES[SH];
   uint32_t v[6];
@@ -98,19 +101,23 @@ struct ShapeVals {
 
  private:
   template <int S>
+  __device__ __forceinline__ uint32_t at(const ShapeArgs &A, uint32_t row) const {
+    return JOIN && A.fk[S] ? __ldg(A.fk[S] + row) : row;
+  }
+  template <int S>
   __device__ __forceinline__ void n1(const ShapeArgs &A, uint32_t row) {
     using T = ShapeSlot<SH, NARROW, S>;
-    if (T::kv && T::filt) v[S] = shape_load<T::w>(A.col[S], row);
+    if (T::kv && T::filt) v[S] = shape_load<T::w>(A.col[S], at<S>(A, row));
   }
   template <int S>
   __device__ __forceinline__ void l1(const ShapeArgs &A, uint32_t row, bool on) {
     using T = ShapeSlot<SH, NARROW, S>;
-    if (T::kv && !T::filt && on) v[S] = shape_load<T::w>(A.col[S], row);
+    if (T::kv && !T::filt && on) v[S] = shape_load<T::w>(A.col[S], at<S>(A, row));
   }
   template <int S>
   __device__ __forceinline__ void f1(const ShapeArgs &A, uint32_t row, bool unc) {
     using T = ShapeSlot<SH, NARROW, S>;
-    if (T::filt && !T::kv && ((A.fmask >> S) & 1u) && unc) v[S] = shape_load<T::w>(A.col[S], row);
+    if (T::filt && !T::kv && ((A.fmask >> S) & 1u) && unc) v[S] = shape_load<T::w>(A.col[S], at<S>(A, row));
   }
   template <int S>
   __device__ __forceinline__ bool c1(const ShapeArgs &A) const {
@@ -135,18 +142,20 @@ struct ShapeVals {
 // no filter reads are loaded only once it has passed its check, which saves
 // their sectors where selected rows are sparse and costs a second memory round
 // trip where they are dense.
-template <int SH, bool NARROW, bool CHK, int GS, int R>
+template <int SH, bool NARROW, bool CHK, int GS, int R, bool JOIN = false>
 __device__ __forceinline__ void shape_rows(const ShapeArgs &A, const uint32_t *q, uint32_t n, bool late,
                                            const GrpCtx &G, int64_t &acc, uint32_t &cnt) {
   const uint32_t lane = threadIdx.x & 31;
-  ShapeVals<SH, NARROW> V[R];
+  ShapeVals<SH, NARROW, JOIN> V[R];
   bool act[R], unc[R];
   uint32_t row[R];
 #pragma unroll
   for (int j = 0; j < R; ++j) {
     const uint32_t i = lane + 32 * j;
     act[j] = i < n;
-    const uint32_t e = act[j] ? q[i] : 0u;
+    // an inactive lane loads row 0, which exists; through a key, a live row (n > 0),
+    // whose key is known to be inside its dimension
+    const uint32_t e = act[j] ? q[i] : (JOIN ? q[0] : 0u);
     row[j] = CHK ? e & 0x7fffffffu : e;
     unc[j] = CHK && (e >> 31);
     V[j].load_now(A, row[j]);

@@ -226,6 +226,11 @@ struct OpNeeds {
   uint32_t kv_mask, filt_mask;
 };
 OpNeeds op_needs(const mb_op &O);
+// A source the op needs has 8-byte elements.
+bool op_reads_wide(const mb_op &O);
+// The group-by strategy of a launch (MB_GRP_AUTO: by the number of groups).
+int pick_gs(uint32_t nr_grp, uint32_t requested);
+mb_status validate_op(const mb_op *op);
 // sure: clauses of the op (bit c) that hold for every row the program selects.
 mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, uint32_t nr_grp, int gs, uint32_t hcap,
                      uint32_t V, uint32_t warps, int64_t *out, uint64_t *nq, uint32_t cps, cudaStream_t st);
