@@ -193,9 +193,9 @@ __global__ void adam_step(float *__restrict__ p, const float *__restrict__ g, fl
 inline unsigned blocks(uint64_t n, unsigned t = 256) { return (unsigned)((n + t - 1) / t); }
 
 // Splits of a weight gradient over n rows: WSPLIT rows each, the splits' sums
-// within 16 MB.
+// within 16 MB and a grid's 65,535 in z.
 uint32_t wgrad_splits(const mb_mlp &M, uint32_t n) {
-  const uint64_t most = std::max<uint64_t>(1, (4u << 20) / M.nparam);
+  const uint64_t most = std::min<uint64_t>(65535, std::max<uint64_t>(1, (4u << 20) / M.nparam));
   return (uint32_t)std::min<uint64_t>((n + WSPLIT - 1) / WSPLIT, most);
 }
 

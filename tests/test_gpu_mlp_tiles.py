@@ -31,3 +31,21 @@ def test_gradients_and_forward(cuda, mb, n, nin, hidden, nout):
         np.testing.assert_allclose(g, wg, rtol=1e-3, atol=1e-5 * np.max(np.abs(wg)))
     finally:
         m.close()
+
+
+def test_gradients_of_more_rows_than_a_grid_has_splits(cuda, mb):
+    """65,536 splits of 128 rows and one row more, the only one with a target: a network
+    this small would take a split per 128 rows, one more than a grid has in z."""
+    from merle_b200 import planner as P
+    n = 65536 * 128 + 1
+    x = np.zeros((n, 1), np.float32)
+    t = np.zeros((n, 1), np.float32)
+    t[-1, 0] = 2
+    m = P.MLP(1, 1, 1, seed=5)
+    try:
+        p = m.get_params()
+        _, g = m.gradients(x, t, np.ones((n, 1), np.float32))
+        _, wg = OM.loss_and_grad(p, x, t, np.ones((n, 1), np.float32), 1, 1, 1)
+        np.testing.assert_allclose(g, wg, rtol=1e-3, atol=1e-5 * np.max(np.abs(wg)))
+    finally:
+        m.close()
