@@ -113,9 +113,7 @@ struct Engine {
   float index_build_ms = 0;
   // query scratch
   int64_t *d_out = nullptr;
-  uint64_t *d_nqual = nullptr;
   int64_t *h_out = nullptr;  // pinned
-  uint64_t *h_nqual = nullptr;
   uint32_t out_cap = 0;
   uint32_t *tmp_bits = nullptr;  // materialisation / row-list scratch
   uint64_t tmp_words = 0;
