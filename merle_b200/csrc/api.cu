@@ -23,7 +23,10 @@ mb_status fail(mb_status st, const char *fmt, ...) {
   return st;
 }
 
+// The error is reported here: the runtime's own record of it is cleared, or the
+// check after the next launch would report it again as that launch's.
 mb_status cuda_fail(cudaError_t e, const char *what) {
+  cudaGetLastError();
   set_error("%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? MB_ERR_OOM : MB_ERR_CUDA;
 }
@@ -59,7 +62,10 @@ cudaMemPool_t scratch_pool() {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
     cudaMemPool_t p = nullptr;
-    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
     uint64_t keep = ~0ull;
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
     pools[dev] = p;
@@ -76,7 +82,10 @@ uint32_t *device_error_word() {
   if ((int)words.size() <= dev) words.resize(dev + 1, nullptr);
   if (!words[dev]) {
     uint32_t *p = nullptr;
-    if (cudaMalloc(&p, 4 * sizeof(uint32_t)) != cudaSuccess) return nullptr;
+    if (cudaMalloc(&p, 4 * sizeof(uint32_t)) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
     cudaMemset(p, 0, 4 * sizeof(uint32_t));
     words[dev] = p;
   }

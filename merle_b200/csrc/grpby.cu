@@ -557,7 +557,10 @@ static uint32_t *seg_scratch(uint64_t nseg) {
     bufs[dev] = nullptr;
     caps[dev] = 0;
     uint64_t cap = nseg < 4096 ? 4096 : nseg;
-    if (cudaMalloc(&bufs[dev], cap * sizeof(uint32_t)) != cudaSuccess) return nullptr;
+    if (cudaMalloc(&bufs[dev], cap * sizeof(uint32_t)) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
     caps[dev] = cap;
   }
   return bufs[dev];
