@@ -98,7 +98,9 @@ void Engine::free_star() {
 mb_status Engine::ensure_out(uint32_t n) {
   if (n <= out_cap) return MB_OK;
   uint32_t cap = std::max<uint32_t>(n, 8192);
+  out_cap = 0;  // until both buffers are there
   free_one(allocs, d_out);
+  d_out = nullptr;
   if (h_out) cudaFreeHost(h_out);
   h_out = nullptr;
   MB_CHECK(alloc((void **)&d_out, ((size_t)cap + 1) * 8));
@@ -109,6 +111,7 @@ mb_status Engine::ensure_out(uint32_t n) {
 
 mb_status Engine::ensure_tmp(uint64_t words) {
   if (words <= tmp_words) return MB_OK;
+  tmp_words = 0;
   free_one(allocs, tmp_bits);
   tmp_bits = nullptr;
   MB_CHECK(alloc((void **)&tmp_bits, words * 4));
@@ -118,6 +121,7 @@ mb_status Engine::ensure_tmp(uint64_t words) {
 
 mb_status Engine::ensure_rows(uint64_t n) {
   if (n <= rows_cap) return MB_OK;
+  rows_cap = 0;
   free_one(allocs, rows);
   rows = nullptr;
   MB_CHECK(alloc((void **)&rows, n * 4));
@@ -1727,6 +1731,7 @@ extern "C" mb_status mb_engine_query_batch(mb_engine *e, const mb_query *qs, uin
   MB_CUDA(cudaSetDevice(E.device));
   const uint64_t total = mb_queries_layout(qs, n, nullptr);
   if (E.bout_cap < total + n) {
+    E.bout_cap = 0;
     free_one(E.allocs, E.bout);
     E.bout = nullptr;
     MB_CHECK(E.alloc((void **)&E.bout, (total + n) * 8));
@@ -1833,6 +1838,7 @@ extern "C" mb_status mb_engine_tune_batch(mb_engine *e, const mb_query *qs, uint
   if (reps == 0) reps = 3;
   const uint64_t total = mb_queries_layout(qs, n, nullptr);
   if (E.bout_cap < total + n) {
+    E.bout_cap = 0;
     free_one(E.allocs, E.bout);
     E.bout = nullptr;
     MB_CHECK(E.alloc((void **)&E.bout, (total + n) * 8));

@@ -201,6 +201,7 @@ uint32_t wgrad_splits(const mb_mlp &M, uint32_t n) {
 
 mb_status ensure(mb_mlp &M, uint32_t n) {
   if (n <= M.cap) return MB_OK;
+  M.cap = 0;  // until every buffer is there
   float **bufs[] = {&M.x, &M.t, &M.mk, &M.h1, &M.h2, &M.y, &M.dy, &M.d2, &M.d1, &M.part};
   for (float **b : bufs) {
     cudaFree(*b);
