@@ -410,11 +410,13 @@ mb_status fused_tma(const DevPrg &P, const mb_op &O, uint32_t nr_grp, int gs, ui
 }
 
 // ------------------------------------------------- warp-independent kernel
-bool fused_warp_applies(const DevPrg &P, const mb_op &O) {
+bool fused_warp_applies(const DevPrg &P, const mb_op &O, size_t grp_bytes, uint32_t warps) {
   if (P.nrows == 0 || P.nrows >= (1ull << 31)) return false;  // (bit 31 of a queued row: uncertain)
   for (uint32_t s = 0; s < O.nsrc; ++s)
     if (O.src[s].width > 4) return false;
-  return true;
+  // beside a group table near the limit (shared tables of 24,700 groups and more, on
+  // request) a general program's row list of 2 or 4 KB a warp may fit where a queue does not
+  return P.cnf || fw_smem(grp_bytes, warps) + FW_STATIC <= (size_t)dev_info().max_smem_optin;
 }
 
 template <int V, bool CHK, int GS>
@@ -488,7 +490,7 @@ mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, 
   // 120M rows 997 / 879 / 871 us; a 24-query spanning mix, 60M rows 1,735 /
   // 1,496 / 1,555 us; the 64-query spanning mix, 600M rows - / 43.8 / 41.1 ms.
   if (V == 0) V = P.nrows < 4000000 ? 1 : P.nrows < 200000000 ? 2 : 4;
-  if (warps == 0 || warps > 8) warps = 8;  // FW_THREADS bounds the block
+  warps = fw_warps(warps);
   if (!vec4) V = 1;                        // unaligned bitmaps: word loads
   const bool chk = P.chk != 0;
   ShapeArgs A;

@@ -22,6 +22,12 @@ namespace mb {
 
 constexpr uint32_t FW_THREADS = 256;
 constexpr uint32_t FW_QCAP = 32 * 32 + 64;  // one 32-word chunk + fewer than 64 pending rows
+constexpr size_t FW_STATIC = 64 * 8;        // shared memory of the final reduction
+// Warps of a CTA, and its dynamic shared memory beside grp_bytes of group table.
+inline uint32_t fw_warps(uint32_t asked) { return asked == 0 || asked > FW_THREADS / 32 ? FW_THREADS / 32 : asked; }
+inline size_t fw_smem(size_t grp_bytes, uint32_t warps) {
+  return ((grp_bytes + 15) & ~(size_t)15) + (size_t)fw_warps(warps) * FW_QCAP * 4;
+}
 // Selected rows of a 1,024-row chunk below which an uncertain row's value
 // columns wait for its check (shape_rows): below about one row in eight most
 // rows have a 32-byte sector to themselves, so a failing row's sectors are
@@ -150,7 +156,7 @@ __device__ __forceinline__ void fw_compact(const DR &dr, uint32_t *queue, uint32
 template <int V, bool CHK, int GS, bool CNF, class DR>
 __device__ __forceinline__ void fused_warp_body(const DevPrg &P, const DR &dr, uint32_t nr_grp, uint32_t hcap,
                                                 unsigned long long *out, unsigned long long *nqual, uint8_t *smem) {
-  __shared__ uint64_t red[64];
+  __shared__ uint64_t red[FW_STATIC / 8];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const size_t gbytes = (grp_smem_bytes(GS, nr_grp, hcap) + 15) & ~(size_t)15;
   const GrpCtx G = grp_init<GS>(smem, nr_grp, hcap, out);
@@ -197,7 +203,7 @@ fused_shape_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ Sha
 template <typename K, typename... Args>
 mb_status fw_launch(K kern, uint32_t V, uint64_t nwords, size_t gbytes, uint32_t warps, uint32_t cps, cudaStream_t st,
                     Args &&...args) {
-  const size_t smem = ((gbytes + 15) & ~(size_t)15) + (size_t)warps * FW_QCAP * 4;
+  const size_t smem = fw_smem(gbytes, warps);
   const DevInfo &di = dev_info();
   if (smem > (size_t)di.max_smem_optin) return fail(MB_ERR_INVALID, "fused: %zu bytes of shared memory", smem);
   MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -498,7 +498,7 @@ mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_
   if (L.words_per_lane != 0 && L.words_per_lane != 1 && L.words_per_lane != 2 && L.words_per_lane != 4)
     return fail(MB_ERR_INVALID, "mb_vprg_grpby: words_per_lane %u", L.words_per_lane);
   const uint32_t hcap = DEFAULT_HCAP;
-  if (L.staging == MB_STAGE_AUTO && fused_warp_applies(P, *op))
+  if (L.staging == MB_STAGE_AUTO && fused_warp_applies(P, *op, grp_smem_bytes(gs, nr_grp, hcap), L.warps_per_cta))
     return fused_warp(P, v4, *op, sure, nr_grp, gs, hcap, L.words_per_lane, L.warps_per_cta, out, nqual, L.ctas_per_sm, st);
   if (L.staging == MB_STAGE_TMA && fused_tma_applies(P, v4, *op)) {
     const mb_status r = fused_tma(P, *op, nr_grp, gs, hcap, L.words_per_lane, out, nqual, L.ctas_per_sm, st);

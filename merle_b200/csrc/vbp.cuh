@@ -218,8 +218,9 @@ mb_status fused_tma(const DevPrg &P, const mb_op &O, uint32_t nr_grp, int gs, ui
 
 namespace mb {
 // The warp-independent kernel (fused.cu): any program over an op whose sources
-// have at most 4 bytes.
-bool fused_warp_applies(const DevPrg &P, const mb_op &O);
+// have at most 4 bytes.  grp_bytes: of the group table in shared memory; warps: as
+// asked for in the launch.
+bool fused_warp_applies(const DevPrg &P, const mb_op &O, size_t grp_bytes, uint32_t warps);
 // Which op sources every row needs (keys, value) and which only uncertain
 // rows need (filter terms).
 struct OpNeeds {
