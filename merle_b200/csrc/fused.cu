@@ -411,7 +411,8 @@ mb_status fused_tma(const DevPrg &P, const mb_op &O, uint32_t nr_grp, int gs, ui
 
 // ------------------------------------------------- warp-independent kernel
 bool fused_warp_applies(const DevPrg &P, const mb_op &O, size_t grp_bytes, uint32_t warps) {
-  if (P.nrows == 0 || P.nrows >= (1ull << 31)) return false;  // (bit 31 of a queued row: uncertain)
+  // with candidate checks, bit 31 of a queued row says that it is uncertain
+  if (P.nrows == 0 || P.nrows >= (P.chk ? 1ull << 31 : 1ull << 32)) return false;
   for (uint32_t s = 0; s < O.nsrc; ++s)
     if (O.src[s].width > 4) return false;
   // beside a group table near the limit (shared tables of 24,700 groups and more, on

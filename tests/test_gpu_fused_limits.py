@@ -47,3 +47,39 @@ def test_general_program_beside_a_large_shared_table(mb, cuda, words, groups, of
     out, nq = D.vprg_grpby(prg, op, groups, launch(grp_strategy=abi.GRP_SHARED, words_per_lane=words))
     np.testing.assert_array_equal(D.to_host(out, np.int64), want)
     assert int(D.to_host(nq, np.uint64)[0]) == len(rows)
+
+
+@pytest.mark.parametrize("chk", [False, True])
+@pytest.mark.parametrize("instrs", [[(abi.ORM, 0, 0, 0)], [(abi.ORM, 0, 0, 0), (abi.ORM, 0, 1, 0)]])
+def test_rows_past_2_31(mb, cuda, chk, instrs):
+    """Row numbers of 32 bits, conjunctive and general programs.  Without candidate checks the
+    warp-independent kernel takes them: 24,000 groups fit beside its queues (192,000 +
+    34,816 bytes) and not beside the general kernel's lists of four words a lane
+    (65,536); with checks the general kernel does, with a smaller table."""
+    n = (1 << 31) + 100_003
+    groups = 1000 if chk else 24_000
+    words = (n + 31) // 32
+    bm = [D.empty(words + 8, 4, zero=True) for _ in range(2)]
+    r = np.random.default_rng(7)
+    rows = [np.unique(np.concatenate([r.integers(0, n, 3000), np.array(x)])) for x in
+            ([0, (1 << 31) - 1, 1 << 31, n - 1], [5, (1 << 31) + 77, n - 2])]
+    for b, q in zip(bm, rows):
+        w, at = np.unique(q // 32, return_inverse=True)
+        v = np.zeros(len(w), np.uint32)
+        np.bitwise_or.at(v, at, np.uint32(1) << (q % 32).astype(np.uint32))
+        b[cuda.from_numpy(w).cuda()] = cuda.from_numpy(v.view(np.int32)).cuda()
+    col = D.empty(n, 1, zero=True)
+    sel = rows[0] if len(instrs) == 1 else np.union1d(rows[0], rows[1])
+    val = (sel % 251).astype(np.uint8)
+    col[cuda.from_numpy(sel).cuda()] = cuda.from_numpy(val).cuda()
+    cols = [ops.Col(middle=[b]) for b in bm]
+    if chk:  # the first operand's rows are candidates of 10 <= value < 200
+        cols[0] = ops.Col(leftmost=bm[0])
+    prg = ops.Vprg(n, cols, instrs).to_c()
+    op = ops.Op(srcs=[ops.Src(col)], clauses=[[(0, 10, 200)]], keys=[(0, abi.X_ID, 1, 0, 1)], vkind=abi.V_ONE).to_c()
+    sure = np.isin(sel, rows[1]) if len(instrs) == 2 else np.zeros(len(sel), bool)
+    keep = (sure | ((val >= 10) & (val < 200))) if chk else np.ones(len(sel), bool)
+    want = np.bincount(val[keep], minlength=groups)
+    out, nq = D.vprg_grpby(prg, op, groups, launch(grp_strategy=abi.GRP_SHARED))
+    np.testing.assert_array_equal(D.to_host(out, np.int64), want)
+    assert int(D.to_host(nq, np.uint64)[0]) == int(keep.sum())
