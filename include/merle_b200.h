@@ -910,8 +910,9 @@ MB_API mb_status mb_wah_op(uint32_t op, const uint32_t *a, uint64_t na, const ui
  * forms, wahAndExpl ...); MB_WAH_DIRECT cuts the runs of both streams at the
  * union of their word boundaries and combines each piece whole, never
  * expanding (wahAnd / wahOr / wahXor, merle/wahGpuDirect.cu); MB_WAH_AUTO
- * (mb_wah_op) takes the direct form when na + nb < ngroups / 2048.  Both give
- * the same canonical stream. */
+ * (mb_wah_op) takes the direct form where it is expected to be the faster: few
+ * words next to the groups, and some millions of groups.  Both give the same
+ * canonical stream. */
 typedef enum mb_wah_method { MB_WAH_AUTO = 0, MB_WAH_EXPLICIT = 1, MB_WAH_DIRECT = 2 } mb_wah_method;
 MB_API mb_status mb_wah_op_ex(uint32_t op, const uint32_t *a, uint64_t na, const uint32_t *b, uint64_t nb,
                               uint64_t ngroups, uint32_t method, uint32_t *out, uint64_t capacity,

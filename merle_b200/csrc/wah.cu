@@ -35,6 +35,7 @@
 // two 600M-row bitmaps of 1 % non-zero words: 702 -> 324 us.
 #include <string.h>
 #include <stdio.h>
+#include <algorithm>
 #include <vector>
 #include "common.cuh"
 
@@ -54,11 +55,26 @@ constexpr uint32_t WAH_MAGIC = 0x44f8a1efu;
 // Blocks up to which a pass sums the block counts before its own itself instead
 // of after a scan launch (at most 64 KB of counts read by each).
 constexpr uint64_t DIRECT_SUM = 8192;
-// mb_wah_op's automatic choice: groups per stream word from which the direct form
-// is taken.  19.4M groups, both streams' words against the time of the explicit /
-// direct form: 747K 139 / 250 us, 76K 138 / 165, 7.6K 152 / 144, 746 164 / 90; at
-// 645K groups and fewer the explicit form is never behind.
-constexpr uint64_t DIRECT_RATIO = 2048;
+// mb_wah_op's automatic choice: the direct form where it is expected to be the faster,
+// from what the forms take in ns.  The explicit one's time grows with the groups, the
+// direct one's with the words of both streams: steeply while its few blocks wait for their
+// binary searches, slowly from 4,000 words on.  Explicit / direct in us, by
+// groups (across) and words (down):
+//              0.6M      6.5M       19.4M       30M        58M      300M
+//     200    57 / 79   85 / 79    123 / 79   164 / 82   250 / 80   984 / 82
+//   2,000    55 / 136  88 / 137   147 / 135  193 / 138  288 / 137  1,123 / 137
+//   6,000    57 / 222  72 / 221   145 / 227  193 / 224  290 / 223  1,129 / 224
+//    200K    59 / 265  71 / 264   113 / 267  155 / 270  239 / 268  976 / 268
+//      6M                                   177 / 1,309            977 / 1,315
+// (The explicit form is slower by 30 % while most of its blocks hold a word or two.)  The
+// form taken is within 11 % of the faster one at each of 185 points measured from 20K to
+// 300M groups and 10 to 6M words; a word for every 2,048 groups, the line before, was off by
+// up to 3.6 times (19.4M groups and 6,000 words: 227 us instead of 145).
+inline bool direct_pays(uint64_t words, uint64_t groups) {
+  const uint64_t expl = 56000 + groups * (2048 * words < groups ? 45 : 32) / 10000;
+  const uint64_t direct = 76000 + std::min<uint64_t>(36 * words, 150000) + words * 2 / 11;
+  return direct < expl;
+}
 
 __device__ __forceinline__ uint32_t kind_of(uint32_t v) { return v == 0 ? 0u : v == LIT ? 1u : 2u; }
 __device__ __forceinline__ uint64_t word_groups(uint32_t w) { return (w & FILL) ? (w & CNT) : 1u; }
@@ -1031,9 +1047,9 @@ extern "C" mb_status mb_wah_op_ex(uint32_t op, const uint32_t *a, uint64_t na, c
                                         (unsigned long long)ngroups);
   if (ngroups == 0) return MB_OK;
   cudaStream_t st = as_stream(stream);
-  // direct when the streams are short next to the groups: its work follows the
-  // words (with binary searches per piece), the other form's the groups
-  if (method == MB_WAH_DIRECT || (method == MB_WAH_AUTO && DIRECT_RATIO * (na + nb) < ngroups))
+  // the direct form's work follows the words (with binary searches per piece), the
+  // other form's the groups
+  if (method == MB_WAH_DIRECT || (method == MB_WAH_AUTO && direct_pays(na + nb, ngroups)))
     return direct_op(op, a, na, b, nb, ngroups, out, capacity, nwords, st);
   // the encoder on the groups of both streams, expanded block by block (their
   // bit order is immaterial: both sides and the result keep their own)

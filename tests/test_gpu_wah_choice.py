@@ -1,0 +1,48 @@
+"""mb_wah_op's automatic choice between its two forms, well off the line between them:
+no slower than the faster of the two, and the same stream."""
+from __future__ import annotations
+
+import ctypes as C
+import time
+
+import numpy as np
+import pytest
+
+from merle_b200 import abi, check, device as D
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("groups,words", [(645_000, 100), (6_500_000, 2000), (19_400_000, 6000), (14_000_000, 100),
+                                          (58_000_000, 2000)])
+def test_automatic_form(mb, cuda, groups, words):
+    """Measured at these points the forms differ by 1.4 to 2.1 times; 1.2 parts
+    them and the scatter of the least of 60 calls."""
+    L = D.lib()
+    n = groups * 31
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(words)
+    st = []
+    for _ in range(2):
+        b = cuda.zeros((n + 31) // 32, dtype=cuda.int32, device="cuda")
+        b[cuda.randint(0, b.numel() - 1, (words // 4,), device="cuda", generator=g)] = 1
+        s, k = D.empty(words, 4), C.c_uint64(0)
+        check(L.mb_wah_encode(b.data_ptr(), n, abi.WAH_LSB, s.data_ptr(), words, C.byref(k), D.stream_ptr()))
+        st.append((s, k.value))
+    assert words // 2 < st[0][1] + st[1][1] <= 2 * words
+    (a, na), (b, nb) = st
+    best, out = {}, {}
+    o, k = D.empty(groups, 4), C.c_uint64(0)  # holds any stream of these groups
+    for rep in range(60):
+        for method in (abi.WAH_AUTO, abi.WAH_EXPLICIT, abi.WAH_DIRECT):
+            cuda.cuda.synchronize()
+            t = time.perf_counter()
+            check(L.mb_wah_op_ex(1, a.data_ptr(), na, b.data_ptr(), nb, groups, method, o.data_ptr(), o.numel(),
+                                 C.byref(k), D.stream_ptr()))
+            cuda.cuda.synchronize()
+            best[method] = min(best.get(method, 1e9), time.perf_counter() - t)
+            if rep == 0:
+                out[method] = D.to_host(o[:k.value], np.uint32)
+    for method in (abi.WAH_EXPLICIT, abi.WAH_DIRECT):
+        np.testing.assert_array_equal(out[abi.WAH_AUTO], out[method])
+    assert best[abi.WAH_AUTO] <= 1.2 * min(best[abi.WAH_EXPLICIT], best[abi.WAH_DIRECT]), best
