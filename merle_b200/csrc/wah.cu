@@ -67,7 +67,7 @@ constexpr uint64_t DIRECT_SUM = 8192;
 //    200K    59 / 265  71 / 264   113 / 267  155 / 270  239 / 268  976 / 268
 //      6M                                   177 / 1,309            977 / 1,315
 // (The explicit form is slower by 30 % while most of its blocks hold a word or two.)  The
-// form taken is within 11 % of the faster one at each of 185 points measured from 20K to
+// form taken is within 15 % of the faster one at each of 185 points measured from 20K to
 // 300M groups and 10 to 6M words; a word for every 2,048 groups, the line before, was off by
 // up to 3.6 times (19.4M groups and 6,000 words: 227 us instead of 145).
 inline bool direct_pays(uint64_t words, uint64_t groups) {
