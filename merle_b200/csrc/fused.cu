@@ -486,19 +486,24 @@ int shape_of(const mb_op &O, uint32_t nr_grp, uint32_t sure, ShapeArgs *A, bool 
 
 mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, uint32_t nr_grp, int gs, uint32_t hcap,
                      uint32_t V, uint32_t warps, int64_t *out, uint64_t *nq, uint32_t cps, cudaStream_t st) {
-  // Words a lane: wider tiles mean fewer, wider loads and fewer warps at work.
-  // Device time at V = 1 / 2 / 4: 13 SSB queries, 1M rows 179 / 185 / 189 us,
-  // 120M rows 997 / 879 / 871 us; a 24-query spanning mix, 60M rows 1,735 /
-  // 1,496 / 1,555 us; the 64-query spanning mix, 600M rows - / 43.8 / 41.1 ms.
-  if (V == 0) V = P.nrows < 4000000 ? 1 : P.nrows < 200000000 ? 2 : 4;
-  warps = fw_warps(warps);
-  if (!vec4) V = 1;                        // unaligned bitmaps: word loads
   const bool chk = P.chk != 0;
   ShapeArgs A;
   bool narrow = false;
   const int sh = gs == GS_HASH || !P.cnf ? -1 : shape_of(O, nr_grp, sure, &A, &narrow);
   // a compiled op: one group in a register (shape 1), or several in a table
-  if (sh >= 0 && (sh == 0 ? gs == GS_SCALAR : gs != GS_SCALAR && nr_grp >= GRP_DIRECT_MIN)) {
+  const bool compiled = sh >= 0 && (sh == 0 ? gs == GS_SCALAR : gs != GS_SCALAR && nr_grp >= GRP_DIRECT_MIN);
+  // Words a lane: wider tiles mean fewer, wider loads and fewer warps at work.
+  // Device time at V = 1 / 2 / 4: 13 SSB queries, 1M rows 179 / 185 / 189 us,
+  // 120M rows 997 / 879 / 871 us; a 24-query spanning mix, 60M rows 1,735 /
+  // 1,496 / 1,555 us; the 64-query spanning mix, 600M rows - / 43.8 / 41.1 ms.
+  // An interpreted op never takes four: 240M rows, 256 groups, a chain of one bitmap
+  // over a third of the rows 794 / 965 / 1,481 us, of three over 2 % 425 / 457 /
+  // 552, an OR of three over 30 % 551 / 628 / 1,730; a chain of three over 0.1 %
+  // gains 8 % by it (67.6 / 62.6).
+  if (V == 0) V = P.nrows < 4000000 ? 1 : !compiled || P.nrows < 200000000 ? 2 : 4;
+  warps = fw_warps(warps);
+  if (!vec4) V = 1;                        // unaligned bitmaps: word loads
+  if (compiled) {
     const ShapeLaunch L{nr_grp, V, warps, cps, gs, narrow, reinterpret_cast<unsigned long long *>(out),
                         reinterpret_cast<unsigned long long *>(nq), st};
     switch (sh) {
