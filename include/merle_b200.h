@@ -199,8 +199,10 @@ typedef struct mb_launch {
 } mb_launch;
 
 typedef enum mb_staging {
-  MB_STAGE_AUTO = 0,    /* conjunctive programs: warp-independent tiles with all
-                           operand loads batched; others: MB_STAGE_DIRECT */
+  MB_STAGE_AUTO = 0,    /* warp-independent tiles with all operand loads batched:
+                           conjunctive programs, and general ones where they are
+                           the faster, over sources of up to 4 bytes; others:
+                           MB_STAGE_DIRECT */
   MB_STAGE_DIRECT = 1,  /* the instruction interpreter with per-thread loads */
   MB_STAGE_TMA = 2      /* every operand tile staged in shared memory by TMA
                            bulk copies, double-buffered per CTA */

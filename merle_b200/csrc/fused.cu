@@ -218,20 +218,44 @@ __device__ __forceinline__ void compact_chunk(const mb_op &O, const OpNeeds &N, 
   __syncwarp();
 }
 
-// Any op as the warp-independent kernel's drain (fused_warp.cuh).
+// Any op as the warp-independent kernel's drain (fused_warp.cuh): n queued rows, of a
+// 1,024-row chunk with `rows` selected ones.  Sparse rows wait for their sectors, and
+// drain64 has two rows' loads in flight a lane; dense ones share sectors, and the
+// instructions count: op_eval needs fewer, a row a lane.  120M rows without checks, 256
+// groups, two words a lane: an OR over 30 % of the rows 328 -> 230 us, a chain over a third
+// 488 -> 344, an OR over 0.5 % 89 -> 88.  From 16 rows a chunk on; 32 and 48 are slower by up to
+// 1.2 and 1.4 times where the chunks of a table lie on both sides (an OR over 6 %, 240M
+// rows: 190 us at 16, 228, 273).
+// With candidate checks drain64 alone: both in one kernel make the sparse cases 3 to 20 %
+// slower, and op_eval on rows that fail their checks takes up to 1.46 times as long.
+constexpr uint32_t ANY_DENSE = 16;
 template <bool CHK, int GS>
 struct AnyDrain {
   const mb_op &O;
   OpNeeds N;
   uint32_t nr_grp;
-  __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, bool, const GrpCtx &G, int64_t &acc,
+  __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, uint32_t rows, const GrpCtx &G, int64_t &acc,
                                         uint32_t &cnt) const {
-    drain64<CHK ? DR_FLAG : DR_NOCHK, GS>(O, N, q, n, nr_grp, G, acc, cnt);
+    if (CHK || rows < ANY_DENSE) {
+      drain64<CHK ? DR_FLAG : DR_NOCHK, GS>(O, N, q, n, nr_grp, G, acc, cnt);
+      return;
+    }
+#pragma unroll 1
+    for (uint32_t i = threadIdx.x & 31; i < 64; i += 32) {
+      int64_t val = 0;
+      uint32_t grp = 0;
+      const bool kept = i < n && op_eval(O, q[i], false, nr_grp, val, grp);
+      cnt += kept ? 1u : 0u;
+      aggregate<GS>(G, kept, grp, val, acc);
+    }
   }
 };
 
+// Without checks the CTAs an SM are named (64 registers a thread): left alone, the compiler
+// takes 48 for most and spills, sparse programs up to 12 % slower (24M rows, an OR over
+// 0.5 %: 21.8 -> 19.4 us).
 template <int V, bool CHK, int GS, bool CNF>
-__global__ void __launch_bounds__(FW_THREADS)
+__global__ void __launch_bounds__(FW_THREADS, CHK ? 0 : 4)
 fused_warp_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ mb_op O, OpNeeds N, uint32_t nr_grp,
                   uint32_t hcap, unsigned long long *__restrict__ out, unsigned long long *__restrict__ nqual) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -427,7 +451,10 @@ static mb_status launch_fw(const DevPrg &P, const mb_op &O, uint32_t nr_grp, uin
     return fw_launch(kern, V, P.nwords, grp_smem_bytes(GS, nr_grp, hcap), warps, cps, st, P, O, op_needs(O), nr_grp,
                      hcap, reinterpret_cast<unsigned long long *>(out), reinterpret_cast<unsigned long long *>(nq));
   };
-  return P.cnf ? go(fused_warp_kernel<V, CHK, GS, true>) : go(fused_warp_kernel<V, CHK, GS, false>);
+  if constexpr (V < 4) {  // (general programs of four words run in the general kernel)
+    if (!P.cnf) return go(fused_warp_kernel<V, CHK, GS, false>);
+  }
+  return go(fused_warp_kernel<V, CHK, GS, true>);
 }
 
 template <int V, bool CHK>
@@ -496,11 +523,12 @@ mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, 
   // Device time at V = 1 / 2 / 4: 13 SSB queries, 1M rows 179 / 185 / 189 us,
   // 120M rows 997 / 879 / 871 us; a 24-query spanning mix, 60M rows 1,735 /
   // 1,496 / 1,555 us; the 64-query spanning mix, 600M rows - / 43.8 / 41.1 ms.
-  // An interpreted op never takes four: 240M rows, 256 groups, a chain of one bitmap
-  // over a third of the rows 794 / 965 / 1,481 us, of three over 2 % 425 / 457 /
-  // 552, an OR of three over 30 % 551 / 628 / 1,730; a chain of three over 0.1 %
-  // gains 8 % by it (67.6 / 62.6).
+  // An interpreted op does not take four: 240M rows, 256 groups, a chain over 6 % of
+  // the rows 196 / 189 / 197 us, over a third 640 / 656 / 662, with checks over 6 % 526 / 583
+  // / 734 (over 0.1 % it gains 9 %: 79 / 69 / 63); a general program in this kernel, an OR
+  // over 30 %, - / 429 / 736, with checks 1,510 / 1,609 / 3,367.
   if (V == 0) V = P.nrows < 4000000 ? 1 : !compiled || P.nrows < 200000000 ? 2 : 4;
+  if (V == 4 && !P.cnf) V = 2;             // (no kernel of four; fused_grpby does not ask for it)
   warps = fw_warps(warps);
   if (!vec4) V = 1;                        // unaligned bitmaps: word loads
   if (compiled) {

@@ -144,7 +144,7 @@ __device__ __forceinline__ void fw_compact(const DR &dr, uint32_t *queue, uint32
   __syncwarp();
   while (qn >= 64) {  // drain from the end: the queue's order is irrelevant
     qn -= 64;
-    dr.drain(queue + qn, 64, total < FW_LATE, G, acc, cnt);
+    dr.drain(queue + qn, 64, total, G, acc, cnt);
   }
   __syncwarp();
 }
@@ -176,18 +176,19 @@ __device__ __forceinline__ void fused_warp_body(const DevPrg &P, const DR &dr, u
       if (__any_sync(0xffffffffu, p[k] != 0))
         fw_compact<CHK>(dr, queue, qn, rb + 32 * k, p[k], u[k], G, acc, cnt);
   }
-  if (qn) dr.drain(queue, qn, true, G, acc, cnt);
+  if (qn) dr.drain(queue, qn, 0, G, acc, cnt);
   __syncthreads();
   grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
 }
 
-// A compiled op (shape.cuh) as the kernel's drain.
+// A compiled op (shape.cuh) as the kernel's drain: n queued rows, of a 1,024-row chunk
+// with `rows` selected ones.
 template <int SH, bool NARROW, bool CHK, int GS>
 struct ShapeDrain {
   const ShapeArgs &A;
-  __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, bool late, const GrpCtx &G, int64_t &acc,
+  __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, uint32_t rows, const GrpCtx &G, int64_t &acc,
                                         uint32_t &cnt) const {
-    shape_rows<SH, NARROW, CHK, GS, 2>(A, q, n, late, G, acc, cnt);
+    shape_rows<SH, NARROW, CHK, GS, 2>(A, q, n, rows < FW_LATE, G, acc, cnt);
   }
 };
 

@@ -498,13 +498,27 @@ mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_
   if (L.words_per_lane != 0 && L.words_per_lane != 1 && L.words_per_lane != 2 && L.words_per_lane != 4)
     return fail(MB_ERR_INVALID, "mb_vprg_grpby: words_per_lane %u", L.words_per_lane);
   const uint32_t hcap = DEFAULT_HCAP;
-  if (L.staging == MB_STAGE_AUTO && fused_warp_applies(P, *op, grp_smem_bytes(gs, nr_grp, hcap), L.warps_per_cta))
+  // A general program runs in the kernel that is the faster at the launch's words a lane.
+  // General / warp-independent, us, 120M rows, 256 groups, an OR over 0.5, 6 and 30 % of the
+  // rows, and over a third of them with few to check:
+  //   with checks     one word  211 / 152, 340 / 307, 780 / 761,     309 / 493
+  //                   two       134 / 116, 286 / 303, 785 / 813,     292 / 588
+  //                   four      135 / 168, 424 / 592, 1,320 / 1,590, 523 / 1,560
+  //   without         one       116 / 138, 113 / 136, 192 / 250,     228 / 280
+  //                   two        86 / 88,  113 / 114, 222 / 230,     272 / 262
+  //                   four       99 / 113, 157 / 160, 372 / 389,     480 / 431
+  // Without words of its own: warp-independent with the one or two of fused_warp, but with
+  // checks from 200M rows on general with two (240M rows: 259 / 210, 529 / 563, 1,421 /
+  // 1,593, 636 / 1,154; the general kernel with four 253, 813, 2,562, 1,117).
+  const uint32_t words = v4 ? L.words_per_lane : 1;
+  const bool general = !P.cnf && (words == 4 || (chk ? words == 2 || (words == 0 && P.nrows >= 200000000) : words == 1));
+  if (L.staging == MB_STAGE_AUTO && !general && fused_warp_applies(P, *op, grp_smem_bytes(gs, nr_grp, hcap), L.warps_per_cta))
     return fused_warp(P, v4, *op, sure, nr_grp, gs, hcap, L.words_per_lane, L.warps_per_cta, out, nqual, L.ctas_per_sm, st);
   if (L.staging == MB_STAGE_TMA && fused_tma_applies(P, v4, *op)) {
     const mb_status r = fused_tma(P, *op, nr_grp, gs, hcap, L.words_per_lane, out, nqual, L.ctas_per_sm, st);
     if (r != MB_ERR_UNSUPPORTED) return r;  // else: too many bitmaps to stage, load directly
   }
-  uint32_t V = L.words_per_lane ? L.words_per_lane : 4;
+  uint32_t V = L.words_per_lane ? L.words_per_lane : general ? 2 : 4;
   if (!v4) V = 1;  // unaligned bitmaps: scalar loads
   if (V == 4) return chk ? fused_gs<4, true>(gs, P, *op, nr_grp, hcap, out, nqual, warps, L.ctas_per_sm, st)
                          : fused_gs<4, false>(gs, P, *op, nr_grp, hcap, out, nqual, warps, L.ctas_per_sm, st);

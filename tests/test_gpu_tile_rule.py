@@ -1,5 +1,5 @@
-"""The fused kernel's words a lane where the launch names none: never a number that is
-measured to be much the slower, and the same sums."""
+"""The fused kernels an interpreted op takes, and their words a lane where the launch
+names none: never one that is measured to be much the slower, and the same sums."""
 from __future__ import annotations
 
 import numpy as np
@@ -54,3 +54,70 @@ def test_interpreted_op_on_a_large_table(mb, cuda, chk, instrs):
         np.testing.assert_array_equal(out[name][0], out["direct"][0])
         np.testing.assert_array_equal(out[name][1], out["direct"][1])
     assert best["default"] <= 1.15 * best[2], best
+
+
+@pytest.mark.parametrize("chk", [False, True])
+def test_general_program_no_slower_than_its_other_kernel(mb, cuda, chk):
+    """120M rows, an OR over a third of them, 256 groups: without checks, and with them at
+    two and four words a lane, what is taken is never more than 12 % slower than the general
+    kernel at the same words (evaluating two rows a lane with every source loaded first, it
+    was by 1.5 to 3 times)."""
+    n = 120_000_011
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(4)
+    col = cuda.randint(0, 256, (n,), dtype=cuda.uint8, device="cuda", generator=g)
+    bm, _ = D.bitmap_create(D.src_of(col), n, [0, 40], [64, 80])
+    cols = [ops.Col(middle=[bm[0]], rightmost=bm[1] if chk else None), ops.Col(middle=[bm[1]])]
+    prg = ops.Vprg(n, cols, [(abi.ORM, 0, 0, 0), (abi.ORM, 0, 1, 0)]).to_c()
+    op = ops.Op(srcs=[ops.Src(col)], clauses=[[(0, 0, 70)]], keys=[(0, abi.X_ID, 1, 0, 1)], vkind=abi.V_ONE).to_c()
+
+    def call(words, staging):
+        la = abi.mb_launch()
+        la.words_per_lane, la.staging = words, staging
+        return lambda: D.vprg_grpby(prg, op, 256, la)
+    best, out = timed(cuda, 9, {(w, s): call(w, s) for w in (0, 1, 2, 4) for s in (STAGE_AUTO, STAGE_DIRECT)})
+    for k in best:
+        np.testing.assert_array_equal(out[k][0], out[0, STAGE_DIRECT][0])
+        np.testing.assert_array_equal(out[k][1], out[0, STAGE_DIRECT][1])
+    for w in (2, 4) if chk else (0, 1, 2, 4):
+        assert best[w, STAGE_AUTO] <= 1.12 * best[w, STAGE_DIRECT], (w, best)
+    assert chk or best[0, STAGE_AUTO] <= 1.12 * best[2, STAGE_DIRECT], best
+
+
+@pytest.mark.parametrize("density", [0.004, 16 / 1024, 0.06, 0.5, 1.0])
+@pytest.mark.parametrize("instrs", [[(abi.ORM, 0, 0, 0)], [(abi.ORM, 0, 0, 0), (abi.ORM, 0, 1, 0)]],
+                         ids=["chain", "general"])
+def test_sparse_and_dense_chunks(mb, cuda, instrs, density):
+    """Chunks below, around and above the 16 rows from which rows are evaluated one a lane, full
+    and partial drain batches, a ragged table: every tile width and group strategy against
+    sums taken on the host."""
+    n = 150_007
+    r = np.random.default_rng(int(density * 1000))
+    sel = r.random((2, n)) < np.array([[density], [density / 4]])
+    sel[0, 50_000:60_000] = True  # a dense stretch in any case
+    key, a, b = r.integers(0, 11, n).astype(np.uint8), r.integers(0, 1 << 32, n).astype(np.uint32), \
+        r.integers(0, 1 << 16, n).astype(np.uint16)
+    words = (n + 31) // 32
+    bm = []
+    for q in sel:
+        w = np.zeros(words * 4 + 32, np.uint8)
+        x = np.packbits(q, bitorder="little")
+        w[:len(x)] = x
+        bm.append(D.from_host(w[:len(w) // 4 * 4].view(np.uint32)))
+    rows = sel[0] | sel[1] if len(instrs) == 2 else sel[0]
+    want = np.zeros(11, np.int64)
+    np.add.at(want, key[rows], a[rows].astype(np.int64) * b[rows])
+    prg = ops.Vprg(n, [ops.Col(middle=[x]) for x in bm], instrs).to_c()
+    dev = [D.from_host(x) for x in (key, a, b)]
+    op = ops.Op(srcs=[ops.Src(x) for x in dev], keys=[(0, abi.X_ID, 1, 0, 1)], vkind=abi.V_MUL, va=1, vb=2)
+    one = ops.Op(srcs=[ops.Src(x) for x in dev], vkind=abi.V_MUL, va=1, vb=2).to_c()
+    op = op.to_c()
+    for words_per_lane in (0, 1, 2, 4):
+        for gs in (abi.GRP_AUTO, abi.GRP_SHARED, abi.GRP_GLOBAL, abi.GRP_HASH):
+            la = abi.mb_launch()
+            la.words_per_lane, la.grp_strategy = words_per_lane, gs
+            out, nq = D.vprg_grpby(prg, op, 11, la)
+            np.testing.assert_array_equal(D.to_host(out, np.int64), want, err_msg=f"{words_per_lane} {gs}")
+            assert int(D.to_host(nq, np.uint64)[0]) == int(rows.sum())
+            out, nq = D.vprg_grpby(prg, one, 1, la)
+            assert int(D.to_host(out, np.int64)[0]) == int(want.sum())
