@@ -1,11 +1,13 @@
-"""The fused kernels an interpreted op takes, and their words a lane where the launch
-names none: never one that is measured to be much the slower, and the same sums."""
+"""The fused kernels an op takes, and their words a lane where the launch names none:
+never one that is measured to be much the slower, and the same sums."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
-from merle_b200 import abi, device as D, ops
+from merle_b200 import abi, device as D, ops, workload as WL
+from merle_b200.engine import Engine
+from merle_b200.planner import _run_timed
 
 pytestmark = pytest.mark.gpu
 
@@ -121,3 +123,29 @@ def test_sparse_and_dense_chunks(mb, cuda, instrs, density):
             assert int(D.to_host(nq, np.uint64)[0]) == int(rows.sum())
             out, nq = D.vprg_grpby(prg, one, 1, la)
             assert int(D.to_host(out, np.int64)[0]) == int(want.sum())
+
+
+def test_templates_on_large_tables_take_four_words_a_lane(mb, cuda):
+    """24 random queries, 120M rows: 1,159 us at two words a lane, 1,090 at four (6 %);
+    half of that parts them and the scatter of the least of 9 runs."""
+    e = Engine(0)
+    try:
+        e.gen_star(2, 20, 120_000_000)
+        e.build_index()
+        qs = WL.random_mix(3, 24)
+        out, nq = D.empty(sum(max(1, e.ngroups(q)) for q in qs), 8), D.empty(len(qs), 8)
+        best, sums = {}, {}
+        for _ in range(9):
+            for v in (0, 2, 4):
+                plans = []
+                for _q in qs:
+                    p = abi.mb_plan()
+                    p.kind, p.launch.words_per_lane = abi.PLAN_FUSED, v
+                    plans.append(p)
+                best[v] = min(best.get(v, 1e9), float(_run_timed(e, qs, plans, out, nq).sum()))
+                sums[v] = D.to_host(out, np.int64)
+        for v in (2, 4):
+            np.testing.assert_array_equal(sums[0], sums[v])
+        assert best[0] <= 1.03 * min(best[2], best[4]), best
+    finally:
+        e.close()
