@@ -95,9 +95,9 @@ __device__ __forceinline__ bool eval_row(const mb_op &O, const uint32_t (&v)[MB_
   return true;
 }
 
-// Which queued rows the op's clauses are evaluated on: none, those whose entry has
-// bit 31 set, all (the entry is then the whole row id).
-enum { DR_NOCHK = 0, DR_FLAG = 1, DR_ALL = 2 };
+// Which queued rows the op's clauses are evaluated on: none (the entry is then the whole
+// row id), those whose entry has bit 31 set.
+enum { DR_NOCHK = 0, DR_FLAG = 1 };
 
 // Runs the op over 64 queued rows (two per lane) and aggregates them.
 template <int CHK, int GS>
@@ -107,7 +107,7 @@ __device__ __forceinline__ void drain64(const mb_op &O, const OpNeeds &N, const 
   const uint32_t lane = threadIdx.x & 31;
   const bool ok0 = lane < nrows_avail, ok1 = lane + 32 < nrows_avail;
   const uint32_t e0 = ok0 ? q[lane] : 0u, e1 = ok1 ? q[lane + 32] : 0u;
-  const bool c0 = CHK == DR_ALL || (CHK == DR_FLAG && (e0 >> 31)), c1 = CHK == DR_ALL || (CHK == DR_FLAG && (e1 >> 31));
+  const bool c0 = CHK == DR_FLAG && (e0 >> 31), c1 = CHK == DR_FLAG && (e1 >> 31);
   uint32_t v0[MB_MAXSRC], v1[MB_MAXSRC], bad0, bad1;
   load_row(O, ok0 ? (N.kv_mask | (c0 ? N.filt_mask : 0u)) : 0u, e0 & ROW, v0, bad0);
   load_row(O, ok1 ? (N.kv_mask | (c1 ? N.filt_mask : 0u)) : 0u, e1 & ROW, v1, bad1);

@@ -4,13 +4,15 @@
 // Reference kernels: grpby (primitive.cuh:16-48) and the comparison system's joins
 // (crystal/src/ssb/q21.cu and its siblings).
 //
-// One kernel serves both.  The clauses that are one range on a fact column, and the
-// dimensions with a filter of their own, become screens: a warp takes 1,024 rows, each
+// Compiled ops (shape.cuh), and any op that the clauses on fact columns filter alone or with
+// key bits: the clauses that are one range on a fact column, and the
+// dimensions with a filter of their own, become screens.  A warp takes 1,024 rows, each
 // lane four consecutive rows in each of eight 128-row chunks, and tests the screens one
 // after the other on vector loads; a lane whose four rows all failed loads no more, so
 // a later column's 32-byte sectors without a live row are not fetched.  The surviving
-// rows queue per warp, and full batches of 64 run the rest of the op, with every source of
-// every row loaded together (opdrain.cuh).
+// rows queue per warp, and full batches of 64 run the rest of the op.  Any other op, and
+// small tables, go row by row (join_grpby_kernel): one clause screens, the rows that pass
+// queue, and full warps of them run the op.
 //
 // A dimension's screen is one bit a dimension row (dimension keys are row numbers 0 ..
 // dimsz - 1, so the key itself is a perfect hash): built by one pass over the dimension,
@@ -29,7 +31,6 @@
 #include <string.h>
 #include <algorithm>
 #include "common.cuh"
-#include "opdrain.cuh"
 #include "opeval.cuh"
 #include "shape.cuh"
 #include "vbp.cuh"
@@ -328,37 +329,34 @@ __device__ __forceinline__ void scan_body(uint64_t nrows, const DR &dr, const Sc
   grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
 }
 
-// Any op without the clauses that are screens.  CHK: it still has some.  WIDE: it needs
-// 8-byte sources (op_eval, a row a lane).
-template <int GS, bool CHK, bool WIDE>
+// Any op without the clauses that are screens, a row a lane (CHK: it still has some).
+// Loading every source of two rows together instead: 1.1 to 1.9 times as long on
+// interpreted ops (240M rows, half of them selected, 200 groups: 1,062 us here, 1,464).
+template <int GS, bool CHK>
 struct OpDrain {
   const mb_op &O;
-  OpNeeds N;
   uint32_t nr_grp;
   __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, const GrpCtx &G, int64_t &acc,
                                         uint32_t &cnt) const {
-    if constexpr (!WIDE) {
-      drain64<CHK ? DR_ALL : DR_NOCHK, GS>(O, N, q, n, nr_grp, G, acc, cnt);
-    } else {
-      for (uint32_t i = threadIdx.x & 31; i < 64; i += 32) {
-        bool kept = false;
-        int64_t val = 0;
-        uint32_t grp = 0;
-        if (i < n) kept = op_eval(O, q[i], CHK, nr_grp, val, grp);
-        cnt += kept ? 1u : 0u;
-        aggregate<GS>(G, kept, grp, val, acc);
-      }
+#pragma unroll 1
+    for (uint32_t i = threadIdx.x & 31; i < 64; i += 32) {
+      bool kept = false;
+      int64_t val = 0;
+      uint32_t grp = 0;
+      if (i < n) kept = op_eval(O, q[i], CHK, nr_grp, val, grp);
+      cnt += kept ? 1u : 0u;
+      aggregate<GS>(G, kept, grp, val, acc);
     }
   }
 };
 
-template <int GS, bool CHK, bool WIDE>
+template <int GS, bool CHK>
 __global__ void __launch_bounds__(SC_WARPS * 32, 1)
-scan_kernel(uint64_t nrows, const __grid_constant__ mb_op O, OpNeeds N, const __grid_constant__ ScanArgs A,
-            uint32_t nr_grp, uint32_t grp_bytes, uint32_t stage_words, unsigned long long *__restrict__ out,
+scan_kernel(uint64_t nrows, const __grid_constant__ mb_op O, const __grid_constant__ ScanArgs A, uint32_t nr_grp,
+            uint32_t grp_bytes, uint32_t stage_words, unsigned long long *__restrict__ out,
             unsigned long long *__restrict__ nqual) {
   extern __shared__ __align__(16) uint8_t smem[];
-  scan_body<GS>(nrows, OpDrain<GS, CHK, WIDE>{O, N, nr_grp}, A, nr_grp, grp_bytes, stage_words, out, nqual, smem);
+  scan_body<GS>(nrows, OpDrain<GS, CHK>{O, nr_grp}, A, nr_grp, grp_bytes, stage_words, out, nqual, smem);
 }
 
 // A compiled op all of whose clauses are screens (shape.cuh).
@@ -378,6 +376,127 @@ scan_shape_kernel(uint64_t nrows, const __grid_constant__ ShapeArgs S, const __g
                   unsigned long long *__restrict__ nqual) {
   extern __shared__ __align__(16) uint8_t smem[];
   scan_body<GS>(nrows, ScanShapeDrain<GS, SH, NARROW, JOIN>{S}, A, nr_grp, grp_bytes, stage_words, out, nqual, smem);
+}
+
+// ------------------------------------------------- rows through an interpreted op
+// Clause c alone on one row, as op_eval evaluates it.
+__device__ __forceinline__ bool clause_pass(const mb_op &O, uint32_t c, uint32_t t0, uint32_t row) {
+  bool any = false;
+  for (uint32_t k = 0; k < O.clause_len[c] && !any; ++k) {
+    const mb_term &tm = O.terms[t0 + k];
+    uint64_t v;
+    any = src_value(O.src[tm.src], row, v) && v >= tm.lo && v < tm.hi;
+  }
+  return any;
+}
+
+constexpr uint32_t JOIN_WARPS = 8;
+constexpr uint32_t JQ = 160;  // rows a warp queues between the screen and the op (31 + a 128-row chunk)
+
+// Every row through the op.  A row first meets one clause (`screen`, first
+// term `t0`; none if screen >= nclause), one row per lane; the rows that pass
+// queue per warp, and each full warp of them runs the rest of the op, so the
+// lanes of its loads and branches are all live rows.  The result equals
+// op_eval on every row (the screen is one of the op's own clauses).
+// Four consecutive values of a fact column of SW-byte elements from one
+// vector load (the column 16-byte aligned, rows r .. r+3 inside it, r a
+// multiple of 4).
+template <int SW>
+__device__ __forceinline__ void load4(const void *col, uint64_t r, uint64_t (&v)[4]) {
+  if (SW == 1) {
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(col) + r / 4);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = (w >> (8 * j)) & 0xffu;
+  } else if (SW == 2) {
+    const uint2 w = __ldg(reinterpret_cast<const uint2 *>(col) + r / 4);
+    v[0] = w.x & 0xffffu, v[1] = w.x >> 16, v[2] = w.y & 0xffffu, v[3] = w.y >> 16;
+  } else if (SW == 4) {
+    const uint4 w = __ldg(reinterpret_cast<const uint4 *>(col) + r / 4);
+    v[0] = w.x, v[1] = w.y, v[2] = w.z, v[3] = w.w;
+  } else {
+    const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(col) + r / 2),
+                     b = __ldg(reinterpret_cast<const ulonglong2 *>(col) + r / 2 + 1);
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+  }
+}
+
+template <int GS, int SW>
+__global__ void __launch_bounds__(256, 8)
+join_grpby_kernel(uint64_t nrows, const __grid_constant__ mb_op O, uint32_t nr_grp, uint32_t grp_bytes, uint32_t screen, uint32_t t0, unsigned long long *__restrict__ out,
+                  unsigned long long *__restrict__ nqual) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ uint64_t red[64];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  GrpCtx G = grp_init<GS>(smem, nr_grp, 0, out);
+  uint32_t *queue = reinterpret_cast<uint32_t *>(smem + grp_bytes) + (size_t)warp * JQ;
+  __syncthreads();
+  int64_t acc = 0;
+  uint32_t cnt = 0;
+  uint32_t qn = 0;
+  const uint32_t lt = (1u << lane) - 1u;
+  auto drain = [&](uint32_t m) {  // the last m (<= 32) queued rows through the op
+    bool kept = false;
+    int64_t val = 0;
+    uint32_t grp = 0;
+    if (lane < m) kept = op_eval(O, queue[qn - m + lane], true, nr_grp, val, grp, screen);
+    cnt += kept ? 1u : 0u;
+    aggregate<GS>(G, kept, grp, val, acc);
+    qn -= m;
+    __syncwarp();
+  };
+  const uint64_t nchunks = (nrows + 31) / 32;
+  if (screen >= O.nclause) {  // no screen (or no room for the queues): every row through the op
+    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nchunks; ch += (uint64_t)gridDim.x * nw) {
+      const uint64_t row = ch * 32 + lane;
+      bool kept = false;
+      int64_t val = 0;
+      uint32_t grp = 0;
+      if (row < nrows) kept = op_eval(O, (uint32_t)row, true, nr_grp, val, grp);
+      cnt += kept ? 1u : 0u;
+      aggregate<GS>(G, kept, grp, val, acc);
+    }
+  } else if (SW == 0) {
+    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nchunks; ch += (uint64_t)gridDim.x * nw) {
+      const uint64_t row = ch * 32 + lane;
+      const bool pass = row < nrows && clause_pass(O, screen, t0, (uint32_t)row);
+      const uint32_t bal = __ballot_sync(0xffffffffu, pass);
+      if (pass) queue[qn + __popc(bal & lt)] = (uint32_t)row;
+      qn += __popc(bal);  // at most 31 + 32 < JQ
+      __syncwarp();
+      if (qn >= 32) drain(32);
+    }
+    if (qn) drain(qn);
+  } else {
+    // the screen is one range on a fact column of SW-byte elements: four rows
+    // a lane from one vector load; 128-row chunks, the last one partly by
+    // scalar loads
+    const mb_term &tm = O.terms[t0];
+    const void *col = O.src[tm.src].col;
+    const uint64_t lo = tm.lo, hi = tm.hi, nch4 = (nrows + 127) / 128;
+    for (uint64_t ch = (uint64_t)blockIdx.x * nw + warp; ch < nch4; ch += (uint64_t)gridDim.x * nw) {
+      const uint64_t r = ch * 128 + 4 * lane;
+      uint64_t v[4] = {0, 0, 0, 0};
+      if (ch * 128 + 128 <= nrows) {
+        load4<SW>(col, r, v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (r + j < nrows) v[j] = load_width(col, r + j, SW);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool pass = r + j < nrows && v[j] >= lo && v[j] < hi;
+        const uint32_t bal = __ballot_sync(0xffffffffu, pass);
+        if (pass) queue[qn + __popc(bal & lt)] = (uint32_t)(r + j);
+        qn += __popc(bal);  // at most 31 + 128 < JQ
+      }
+      __syncwarp();
+      while (qn >= 32) drain(32);
+    }
+    if (qn) drain(qn);
+  }
+  __syncthreads();
+  grp_flush<GS>(G, nr_grp, acc, cnt, nqual, red);
 }
 
 // ------------------------------------------------------------------ host
@@ -415,9 +534,66 @@ static mb_status scan_launch(K kern, int gs, const ScanCall &C, ScanArgs &A, con
 
 template <int GS>
 static mb_status scan_gs(const ScanCall &C, const mb_op &O, ScanArgs &A) {
-  if (op_reads_wide(O)) return scan_launch(scan_kernel<GS, true, true>, GS, C, A, O, op_needs(O));
-  return O.nclause ? scan_launch(scan_kernel<GS, true, false>, GS, C, A, O, op_needs(O))
-                   : scan_launch(scan_kernel<GS, false, false>, GS, C, A, O, op_needs(O));
+  return O.nclause ? scan_launch(scan_kernel<GS, true>, GS, C, A, O) : scan_launch(scan_kernel<GS, false>, GS, C, A, O);
+}
+
+// The clause that screens rows in the no-index scan: the first whose terms
+// read fact columns only (one load a row), else the first; nclause if none.
+static uint32_t screen_clause(const mb_op &O, uint32_t *t0) {
+  uint32_t t = 0, first_t = 0;
+  for (uint32_t c = 0; c < O.nclause; ++c) {
+    bool fact = true;
+    for (uint32_t k = 0; k < O.clause_len[c]; ++k)
+      if (O.src[O.terms[t + k].src].fk) fact = false;
+    if (fact) {
+      *t0 = t;
+      return c;
+    }
+    t += O.clause_len[c];
+  }
+  *t0 = first_t;
+  return 0;
+}
+
+template <int GS, int SW>
+static mb_status join_launch(const ScanCall &C, const mb_op &O, uint32_t screen, uint32_t t0) {
+  auto kern = join_grpby_kernel<GS, SW>;
+  const DevInfo &di = dev_info();
+  const size_t gb = (grp_smem_bytes(GS, C.nr_grp, 0) + 15) & ~(size_t)15, qbytes = (size_t)JOIN_WARPS * JQ * 4;
+  // the row queues only where they cost no resident CTA (a large group
+  // table in shared memory can leave no room for them)
+  const size_t cap = (size_t)di.max_smem_optin - 1024;  // room for the kernel's static shared memory
+  MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min(cap, gb + qbytes)));
+  int with = 0, occ = 0;
+  MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, JOIN_WARPS * 32, gb));
+  if (gb + qbytes <= cap) MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&with, kern, JOIN_WARPS * 32, gb + qbytes));
+  if (with < occ) screen = O.nclause;
+  if (occ < 1) return fail(MB_ERR_INVALID, "kernel does not fit on an SM (smem %zu)", gb);
+  const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)di.sms * occ, ceil_div(ceil_div(C.n, 32), JOIN_WARPS));
+  kern<<<grid, JOIN_WARPS * 32, gb + (screen < O.nclause ? qbytes : 0), C.st>>>(C.n, O, C.nr_grp, (uint32_t)gb, screen,
+                                                                               t0, C.out, C.nqual);
+  MB_LAUNCH_CHECK("join_grpby_kernel");
+  return MB_OK;
+}
+
+// The screen's shape picks the kernel: one range on a 16-byte-aligned fact
+// column screens four rows a lane (its width a template argument).
+template <int GS>
+static mb_status join_gs(const ScanCall &C, const mb_op &O) {
+  uint32_t t0 = 0;
+  const uint32_t screen = screen_clause(O, &t0);
+  uint32_t sw = 0;
+  if (screen < O.nclause && O.clause_len[screen] == 1) {
+    const mb_src &s = O.src[O.terms[t0].src];
+    if (!s.fk && (reinterpret_cast<uintptr_t>(s.col) & 15) == 0) sw = s.width;
+  }
+  switch (sw) {
+  case 1: return join_launch<GS, 1>(C, O, screen, t0);
+  case 2: return join_launch<GS, 2>(C, O, screen, t0);
+  case 4: return join_launch<GS, 4>(C, O, screen, t0);
+  case 8: return join_launch<GS, 8>(C, O, screen, t0);
+  default: return join_launch<GS, 0>(C, O, screen, t0);
+  }
 }
 
 template <int SH>
@@ -481,6 +657,21 @@ static mb_status scan_rest(uint64_t n, const mb_op &op, uint32_t done, uint32_t 
     if (sh == 1) return scan_shape<1>(C, S, narrow, join, A);
     if (sh == 2) return scan_shape<2>(C, S, narrow, join, A);
     if (sh == 3) return scan_shape<3>(C, S, narrow, join, A);
+  }
+  // An interpreted op goes through the screens where they are its whole filter, or where a
+  // dimension's key bits are among them, on tables of a tile a warp and more.  Else the row
+  // scan is the faster.  Row scan / screens, us, 240M rows, 200 groups (6M, 300K in
+  // brackets): half of the rows by one range 1,033 / 1,062 (36 / 41, 13 / 22), a tenth
+  // 443 / 365 (26 / 18, 11 / 12), two ranges 1,292 / 646 (43 / 29, 12 / 17); no clause 1,398 /
+  // 1,598 (42 / 60, 20 / 32), a dimension's clause 1,073 / 2,790 (39 / 96, 14 / 53), a range and
+  // a dimension's clause 957 / 1,212 (36 / 44, 12 / 26), an OR 1,435 / 2,987 (47 / 108, 14 /
+  // 53); 60M rows, an 8-byte value or clause 272 / 312 and 264 / 326.
+  if (A.ntab == 0 && (nr == 0 || O.nclause || op_reads_wide(op) || n < (uint64_t)dev_info().sms * SC_WARPS * SC_TILE)) {
+    switch (gs) {
+    case GS_SCALAR: return join_gs<GS_SCALAR>(C, op);
+    case GS_SHARED: return join_gs<GS_SHARED>(C, op);
+    default: return join_gs<GS_GLOBAL>(C, op);
+    }
   }
   switch (gs) {
   case GS_SCALAR: return scan_gs<GS_SCALAR>(C, O, A);
