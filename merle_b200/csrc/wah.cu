@@ -43,8 +43,12 @@ namespace mb {
 namespace {
 
 constexpr uint32_t WT = 256;          // threads of the stream-counting and direct passes
-constexpr uint32_t WI = 16;           // stream words per thread there
+constexpr uint32_t WI = 16;           // stream words of a thread of the counting passes
 constexpr uint32_t WB = WT * WI;      // per block
+// Pieces of a thread of the direct passes, whose binary searches wait for one another (with
+// 16: 1.3 to 1.55 times as long; 600M rows, one word in a thousand: 165 -> 257 us).
+constexpr uint32_t DI = 8;
+constexpr uint32_t DB = WT * DI;      // per block
 constexpr uint32_t GT = 128;          // threads of a group block
 constexpr uint32_t GB = 32 * GT;      // its groups
 constexpr uint32_t GW = 31 * GT;      // its bitmap words
@@ -58,21 +62,21 @@ constexpr uint64_t DIRECT_SUM = 8192;
 // mb_wah_op's automatic choice: the direct form where it is expected to be the faster,
 // from what the forms take in ns.  The explicit one's time grows with the groups, the
 // direct one's with the words of both streams: steeply while its few blocks wait for their
-// binary searches, slowly from 4,000 words on.  Explicit / direct in us, by
+// binary searches, slowly from 2,500 words on.  Explicit / direct in us, by
 // groups (across) and words (down):
 //              0.6M      6.5M       19.4M       30M        58M      300M
-//     200    57 / 79   85 / 79    123 / 79   164 / 82   250 / 80   984 / 82
-//   2,000    55 / 136  88 / 137   147 / 135  193 / 138  288 / 137  1,123 / 137
-//   6,000    57 / 222  72 / 221   145 / 227  193 / 224  290 / 223  1,129 / 224
-//    200K    59 / 265  71 / 264   113 / 267  155 / 270  239 / 268  976 / 268
-//      6M                                   177 / 1,309            977 / 1,315
+//     200    58 / 78   85 / 76    125 / 80   165 / 82   250 / 79   986 / 80
+//   2,000    55 / 133  88 / 133   146 / 134  190 / 136  288 / 135  1,124 / 133
+//   6,000    57 / 145  71 / 145   146 / 148  192 / 147  289 / 147  1,129 / 148
+//    200K    59 / 176  71 / 173   112 / 174  154 / 171  238 / 175  974 / 173
+//      6M                                   178 / 1,227            977 / 1,282
 // (The explicit form is slower by 30 % while most of its blocks hold a word or two.)  The
-// form taken is within 15 % of the faster one at each of 185 points measured from 20K to
+// form taken is within 14 % of the faster one at each of 204 points measured from 20K to
 // 300M groups and 10 to 6M words; a word for every 2,048 groups, the line before, was off by
-// up to 3.6 times (19.4M groups and 6,000 words: 227 us instead of 145).
+// up to 4.7 times (300M groups and 600K words: 960 us instead of 209).
 inline bool direct_pays(uint64_t words, uint64_t groups) {
   const uint64_t expl = 56000 + groups * (2048 * words < groups ? 45 : 32) / 10000;
-  const uint64_t direct = 76000 + std::min<uint64_t>(36 * words, 150000) + words * 2 / 11;
+  const uint64_t direct = 76000 + std::min<uint64_t>(31 * words, 66000) + words * 2 / 11;
   return direct < expl;
 }
 
@@ -894,14 +898,14 @@ __device__ __forceinline__ bool direct_flag(const DirectSrc &D, const uint32_t *
   return k != kind_of(direct_value(D, x0 - 1));
 }
 
-// (3a) output words per block of WB pieces.
+// (3a) output words per block of DB pieces.
 __global__ void __launch_bounds__(WT) wah_direct_count(const DirectSrc D, const uint32_t *m, uint64_t M,
                                                        uint64_t *bcnt) {
   uint32_t c = 0, v;
   uint64_t x;
 #pragma unroll
-  for (uint32_t i = 0; i < WI; ++i)
-    c += direct_flag(D, m, M, (uint64_t)blockIdx.x * WB + i * WT + threadIdx.x, &v, &x) ? 1u : 0u;
+  for (uint32_t i = 0; i < DI; ++i)
+    c += direct_flag(D, m, M, (uint64_t)blockIdx.x * DB + i * WT + threadIdx.x, &v, &x) ? 1u : 0u;
   uint64_t total;
   block_excl_scan<WT, uint64_t>(c, &total);
   if (threadIdx.x == 0) bcnt[blockIdx.x] = total;
@@ -912,10 +916,10 @@ __global__ void __launch_bounds__(WT) wah_direct_write(const DirectSrc D, const 
                                                        const uint64_t *boff, uint32_t *out, uint32_t *pos) {
   uint64_t at = boff[blockIdx.x];
 #pragma unroll 1
-  for (uint32_t i = 0; i < WI; ++i) {
+  for (uint32_t i = 0; i < DI; ++i) {
     uint32_t v = 0, total;
     uint64_t x = 0;
-    const bool f = direct_flag(D, m, M, (uint64_t)blockIdx.x * WB + i * WT + threadIdx.x, &v, &x);
+    const bool f = direct_flag(D, m, M, (uint64_t)blockIdx.x * DB + i * WT + threadIdx.x, &v, &x);
     const uint32_t ex = block_flag_scan(f ? 1u : 0u, &total);
     if (f) {
       const uint32_t k = kind_of(v);
@@ -949,7 +953,7 @@ mb_status direct_op(uint32_t op, const uint32_t *a, uint64_t na, const uint32_t 
   MB_CHECK(sc.get(&m, M));
   wah_direct_merge<<<(unsigned)ceil_div(M, 256), 256, 0, st>>>(D, m);
   MB_LAUNCH_CHECK("wah_direct_merge");
-  const uint64_t nblk = ceil_div(M, WB);
+  const uint64_t nblk = ceil_div(M, DB);
   uint64_t *boff;
   MB_CHECK(sc.get(&boff, nblk + 1));
   wah_direct_count<<<(unsigned)nblk, WT, 0, st>>>(D, m, M, boff);
