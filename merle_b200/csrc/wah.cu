@@ -731,11 +731,12 @@ mb_status block_sums(uint64_t *v, uint64_t n, bool total, bool *scanned, cudaStr
 
 // Scratch of an encoding of nblk group blocks, and of a stream's notes for them.
 struct EncBufs {
-  uint64_t *bcnt, *off;
+  uint64_t *bcnt, *off, *total;
   uint32_t *cont, *groups;
   void plan(Carve &c, uint64_t nblk, bool streams) {
     groups = streams ? c.take<uint32_t>(nblk * GB) : nullptr;
     bcnt = c.take<uint64_t>(nblk + 1), off = c.take<uint64_t>(nblk), cont = c.take<uint32_t>(nblk);
+    total = c.take<uint64_t>(1);
   }
 };
 struct NoteBufs {
@@ -768,12 +769,15 @@ mb_status encode(const EncSrc &S, const EncBufs &B, uint32_t *out, uint64_t capa
     if (*nwords > capacity) return fail(MB_ERR_INVALID, "%s: the stream has %llu words, the output holds %llu", who,
                                         (unsigned long long)*nwords, (unsigned long long)capacity);
   }
-  wah_enc_write<SRC == SRC_STREAMS ? SRC_GROUPS : SRC><<<grid, GT, 0, st>>>(S, B.bcnt, scanned, out, B.off, B.cont, hw);
+  // the words to the host, unless it has them: the call need not wait again then
+  wah_enc_write<SRC == SRC_STREAMS ? SRC_GROUPS : SRC><<<grid, GT, 0, st>>>(S, B.bcnt, scanned, out, B.off, B.cont,
+                                                                           sized ? B.total : hw);
   MB_LAUNCH_CHECK("wah_enc_write");
   if (S.nblk > 1) {
     wah_enc_join<<<(unsigned)ceil_div(S.nblk, 256), 256, 0, st>>>(out, B.off, B.cont, S.nblk);
     MB_LAUNCH_CHECK("wah_enc_join");
   }
+  if (sized) return MB_OK;
   MB_CUDA(cudaStreamSynchronize(st));  // *hw
   *nwords = *hw;
   return MB_OK;
