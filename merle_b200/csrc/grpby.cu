@@ -510,15 +510,19 @@ mb_status fused_grpby(const mb_vprg *p, const mb_op *op, uint32_t nr_grp, int64_
   // Without words of its own: warp-independent with the one or two of fused_warp, but with
   // checks from 200M rows on general with two (240M rows: 259 / 210, 529 / 563, 1,421 /
   // 1,593, 636 / 1,154; the general kernel with four 253, 813, 2,562, 1,117).
+  // With a hash table, general with four where the other takes two (an OR over 2 % of the
+  // rows, 240M: 137 / 223, 60M 41 / 61, 6M 13 / 14; over 30 %, 5,800 / 5,842, 1,586 / 1,511,
+  // 245 / 247; with one, 300K rows, 234 / 71).
   const uint32_t words = v4 ? L.words_per_lane : 1;
-  const bool general = !P.cnf && (words == 4 || (chk ? words == 2 || (words == 0 && P.nrows >= 200000000) : words == 1));
+  const bool general = !P.cnf && ((gs == GS_HASH && words == 0 && P.nrows >= 4000000) || words == 4 ||
+                                  (chk ? words == 2 || (words == 0 && P.nrows >= 200000000) : words == 1));
   if (L.staging == MB_STAGE_AUTO && !general && fused_warp_applies(P, *op, grp_smem_bytes(gs, nr_grp, hcap), L.warps_per_cta))
     return fused_warp(P, v4, *op, sure, nr_grp, gs, hcap, L.words_per_lane, L.warps_per_cta, out, nqual, L.ctas_per_sm, st);
   if (L.staging == MB_STAGE_TMA && fused_tma_applies(P, v4, *op)) {
     const mb_status r = fused_tma(P, *op, nr_grp, gs, hcap, L.words_per_lane, out, nqual, L.ctas_per_sm, st);
     if (r != MB_ERR_UNSUPPORTED) return r;  // else: too many bitmaps to stage, load directly
   }
-  uint32_t V = L.words_per_lane ? L.words_per_lane : general ? 2 : 4;
+  uint32_t V = L.words_per_lane ? L.words_per_lane : general && gs != GS_HASH ? 2 : 4;
   if (!v4) V = 1;  // unaligned bitmaps: scalar loads
   if (V == 4) return chk ? fused_gs<4, true>(gs, P, *op, nr_grp, hcap, out, nqual, warps, L.ctas_per_sm, st)
                          : fused_gs<4, false>(gs, P, *op, nr_grp, hcap, out, nqual, warps, L.ctas_per_sm, st);

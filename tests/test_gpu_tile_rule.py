@@ -86,6 +86,26 @@ def test_general_program_no_slower_than_its_other_kernel(mb, cuda, chk):
     assert chk or best[0, STAGE_AUTO] <= 1.12 * best[2, STAGE_DIRECT], best
 
 
+def test_general_program_with_a_hash_table(mb, cuda):
+    """An OR over 2 % of 120M rows, group sums in a hash table: never more than 12 % slower than the
+    general kernel (in the warp-independent one, 1.5 times as long)."""
+    n = 120_000_011
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(5)
+    col = cuda.randint(0, 256, (n,), dtype=cuda.uint8, device="cuda", generator=g)
+    bm, _ = D.bitmap_create(D.src_of(col), n, [0, 2], [2, 5])
+    prg = ops.Vprg(n, [ops.Col(middle=[x]) for x in bm], [(abi.ORM, 0, 0, 0), (abi.ORM, 0, 1, 0)]).to_c()
+    op = ops.Op(srcs=[ops.Src(col)], keys=[(0, abi.X_ID, 1, 0, 1)], vkind=abi.V_ONE).to_c()
+
+    def call(staging):
+        la = abi.mb_launch()
+        la.grp_strategy, la.staging = abi.GRP_HASH, staging
+        return lambda: D.vprg_grpby(prg, op, 256, la)
+    best, out = timed(cuda, 11, {s: call(s) for s in (STAGE_AUTO, STAGE_DIRECT)})
+    np.testing.assert_array_equal(out[STAGE_AUTO][0], out[STAGE_DIRECT][0])
+    assert best[STAGE_AUTO] <= 1.12 * best[STAGE_DIRECT], best
+
+
 @pytest.mark.parametrize("density", [0.004, 16 / 1024, 0.06, 0.5, 1.0])
 @pytest.mark.parametrize("instrs", [[(abi.ORM, 0, 0, 0)], [(abi.ORM, 0, 0, 0), (abi.ORM, 0, 1, 0)]],
                          ids=["chain", "general"])
