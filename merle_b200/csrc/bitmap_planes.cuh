@@ -1,6 +1,7 @@
 // bitmap_planes.cuh - bitmaps of sorted, disjoint bins by bit planes: the kernel
 // and its launch (bitmap.cu cuts the bins into classes and picks the form).
 #pragma once
+#include <algorithm>
 #include <type_traits>
 #include "common.cuh"
 
@@ -341,7 +342,13 @@ bitmap_planes_kernel(const __grid_constant__ PlaneSpec S, const void *__restrict
   __syncthreads();
 
   const uint64_t nwords = (n + 31) / 32, ntiles = (n + ROWS - 1) / ROWS;
-  const uint32_t cend = S.code0 + S.ncls;
+  // the codes of this CTA: all, or its share where a small table's are split (planes_split)
+  uint32_t cbeg = S.code0 & ~7u, cend = S.code0 + S.ncls;
+  if constexpr (V == 1 && NC == 0) {
+    const uint32_t per = ((cend - cbeg + 7) / 8 + gridDim.y - 1) / gridDim.y * 8;
+    cbeg += blockIdx.y * per;
+    cend = cbeg + per < cend ? cbeg + per : cend;
+  }
   uint32_t nbad = 0;
   for (uint64_t t = (uint64_t)blockIdx.x * BP_WARPS + warp; t < ntiles; t += (uint64_t)gridDim.x * BP_WARPS) {
     const uint64_t row0 = t * ROWS;
@@ -377,7 +384,7 @@ bitmap_planes_kernel(const __grid_constant__ PlaneSpec S, const void *__restrict
           if (whole || w + k < nwords) d[k] = m[k];
       }
     };
-    uint32_t *fine = FINE ? S.out[0] + w : nullptr;
+    uint32_t *fine = FINE ? S.out[0] + w + (cbeg > S.code0 ? cbeg - S.code0 : 0) * stride : nullptr;
     uint32_t acc[NC ? NC : 1][V];
     uint32_t *dst[NC ? NC : 1];
 #pragma unroll
@@ -387,7 +394,7 @@ bitmap_planes_kernel(const __grid_constant__ PlaneSpec S, const void *__restrict
       for (int k = 0; k < V; ++k) acc[l][k] = 0;
     }
 #pragma unroll 1
-    for (uint32_t c0 = S.code0 & ~7u; c0 < cend; c0 += 8) {
+    for (uint32_t c0 = cbeg; c0 < cend; c0 += 8) {
       uint32_t high[2][V];  // the products of planes 3 .. 7, with plane 2 clear and set
 #pragma unroll
       for (int k = 0; k < V; ++k) high[1][k] = 0xffffffffu;
@@ -455,6 +462,16 @@ struct PlanePass {
   LevelsJoinOut jo;
 };
 
+// Shares of a level's codes on a small table, a row of CTAs each, while there are warps without a
+// tile: a warp takes about 0.7 us for 8 codes, and 32 of those one after the other are most
+// of the time of the table (250 bins with their row counts, 300K rows: 31 -> 19 us, as with one
+// shared atomic a row and level).  Join outputs are written by one pass alone.
+inline uint32_t planes_split(const PlanePass &P, uint64_t warps) {
+  if (P.jo.dout || P.jo.bad) return 1;
+  const uint64_t tiles = ceil_div(P.n, bp_rows(1)), groups = ((P.S.code0 & 7u) + P.S.ncls + 7) / 8;
+  return (uint32_t)std::max<uint64_t>(1, std::min(warps / tiles, groups));
+}
+
 template <int W, bool JOIN, int DW, int MODE, int V, bool FINE, int NC>
 mb_status launch_planes_v(const PlanePass &P) {
   auto kern = bitmap_planes_kernel<W, JOIN, DW, MODE, V, FINE, NC>;
@@ -463,10 +480,12 @@ mb_status launch_planes_v(const PlanePass &P) {
   int occ = 0;
   MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, BP_THREADS, smem));
   if (occ < 1) return fail(MB_ERR_INVALID, "bitmap planes: %zu bytes of shared memory", smem);
-  uint64_t grid = (uint64_t)dev_info().sms * occ;
+  const DevInfo &di = dev_info();
+  uint64_t grid = (uint64_t)di.sms * occ;
   const uint64_t need = ceil_div(ceil_div(P.n, bp_rows(V)), BP_WARPS);
   if (grid > need) grid = need;
-  kern<<<(unsigned)grid, BP_THREADS, smem, P.st>>>(P.S, JOIN ? (const void *)P.src->fk : P.src->col,
+  const uint64_t split = V == 1 && NC == 0 ? planes_split(P, (uint64_t)di.sms * occ * BP_WARPS) : 1;
+  kern<<<dim3((unsigned)grid, (unsigned)split), BP_THREADS, smem, P.st>>>(P.S, JOIN ? (const void *)P.src->fk : P.src->col,
                                                    JOIN ? P.src->col : nullptr, P.src->dimsz, P.n, P.stride, P.jo);
   MB_LAUNCH_CHECK("bitmap_planes_kernel");
   return MB_OK;
