@@ -226,13 +226,14 @@ MB_API mb_status mb_bitmap_create(const mb_src *src, uint64_t nrows, const uint6
  * years and months of a date, or the regions and nations of a city).  The
  * reference builds every level with its own create_bin pass
  * (bmpidx_create.cu:14-56, driven per level by ssb/bmpidx-create.cu:56-116);
- * here each row's bin in every level comes from one lookup, so the column is
- * read once.  Level l writes levels[l].nbins bitmaps (bin j = [lo[j], hi[j]))
+ * here each row's bin in every level comes from one lookup, division or search,
+ * so the column is read once.  Level l writes levels[l].nbins bitmaps (bin j = [lo[j], hi[j]))
  * to levels[l].out, `stride_words` apart, and accumulates their popcounts
  * into levels[l].popcounts (device uint64[nbins], or NULL).  src, nrows and
- * the stride as for mb_bitmap_create.  Levels with overlapping or unsorted
- * bins, 255 bins or more, or a value domain too wide for the one-pass lookup
- * run one mb_bitmap_create pass per level instead (same results). */
+ * the stride as for mb_bitmap_create.  The levels' bounds together may cut the
+ * values into at most 254 intervals that lie in a bin; levels of more, and those
+ * with overlapping, unsorted or empty bins, run one mb_bitmap_create pass each
+ * instead (same results). */
 #define MB_MAXLEVELS 4
 typedef struct mb_level {
   const uint64_t *lo, *hi; /* host: nbins bounds each */

@@ -49,7 +49,8 @@ __host__ __device__ constexpr uint32_t bp_rows(int V) { return 1024u * V; }
 // Rows below which a lane takes one word: a warp's latency for a tile (its class
 // loop above all) counts while there are fewer 4,096-row tiles than warps.  V = 1 /
 // V = 4, us: three bin sets of int32 columns, 1M rows 59 / 82, 6M 107 / 106, 24M
-// 291 / 244; the star index, 1M 90 / 146, 10M 223 / 232, 24M 437 / 408.
+// 291 / 244; the star index, 1M 90 / 146, 10M 223 / 232, 24M 437 / 408.  The line lies
+// between the two crossings, 6M for the one, past 10M for the other.
 constexpr uint64_t BP_SMALL = 8000000;
 constexpr uint32_t BP_LUT = 16384;        // values of the lookup table
 constexpr uint32_t BP_MAXCLASS = 254;
@@ -83,7 +84,8 @@ struct LevelsJoinOut {
   unsigned long long *bad;
 };
 
-// 8 x 8 bit transpose of the four byte columns of r: afterwards bit 8 i + j of
+// 8 x 8 bit transpose (by swaps of 4, 2 and 1: Warren, Hacker's Delight, 2nd edition,
+// section 7-3) of the four byte columns of r: afterwards bit 8 i + j of
 // r[b] is bit b of byte i of the former r[j].
 template <int S>
 __device__ __forceinline__ void bit_swap8(uint32_t (&r)[8]) {
@@ -334,7 +336,9 @@ bitmap_planes_kernel(const __grid_constant__ PlaneSpec S, const void *__restrict
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint64_t *bound = reinterpret_cast<uint64_t *>(smem);
   uint8_t *lut = smem + planes_bound(S, MODE);
-  uint32_t *cnt = reinterpret_cast<uint32_t *>(smem + planes_table(S, MODE));  // by code
+  // Rows by code, of this CTA: a column of more than 2^32 rows a CTA (148 of them at
+  // least) would not fit the memory.
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(smem + planes_table(S, MODE));
   constexpr uint32_t ROWS = bp_rows(V);
   uint8_t *tile = smem + planes_table(S, MODE) + 1024 + warp * ROWS;
   for (uint32_t i = tid; i < 256; i += BP_THREADS) cnt[i] = 0;

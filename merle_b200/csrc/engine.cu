@@ -562,7 +562,7 @@ void ssb_build_op(const SsbSrc &S, const mb_query &q, mb_op &out) {
 }
 
 // joins: dimension attributes through their foreign keys even where the
-// engine keeps denormalised copies (the hash-join plan builds its tables
+// engine keeps denormalised copies (the hash-join plan takes its key bits
 // from the dimensions).
 static void build_op(const Engine &E, const mb_query &q, mb_op &out, bool joins = false) {
   SsbSrc S;

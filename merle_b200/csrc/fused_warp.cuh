@@ -12,8 +12,9 @@
 // sector read, 4.3 TB/s), instruction issue above that.  Measured at 600M rows,
 // 4-byte columns, 64 queries of selectivity 1e-6 to 0.5, one launch each: 102.2
 // ms with the op interpreted and 2 words a lane, 43.8 ms compiled, 41.1 ms with 4
-// words a lane; at 46 % selected rows 11.9 -> 2.0 ms.  85 registers and 3 CTAs an
-// SM beat 64 and 4 (spills) by 4 %.
+// words a lane; at 46 % selected rows 11.9 -> 2.0 ms.  Bounding the compiled kernels to 3
+// CTAs an SM (85 registers; they take 56-60, so that 4 fit) beats bounding them to 4 (64, with
+// spills) by 4 %.
 #pragma once
 #include "shape.cuh"
 #include "vbp.cuh"

@@ -192,7 +192,7 @@ __device__ __forceinline__ uint32_t screen_words(const Screen &S, uint64_t r0, u
 
 // A range on a 2-byte column, the two rows of a word at once: clamped to the range, a value
 // outside changes; its 1 is shifted into the half's failures, which a perfect shuffle
-// brings into row order.
+// (Warren, Hacker's Delight, 2nd edition, section 7-2) brings into row order.
 __device__ __forceinline__ uint32_t screen_halves(const Screen &S, uint64_t r0, uint32_t live, bool full) {
   static_assert(SC_CHUNKS == 8, "16 words of two rows");
   const uint32_t lo = (uint32_t)S.lo * 0x10001u, hi = (uint32_t)(S.lo + S.span) * 0x10001u;

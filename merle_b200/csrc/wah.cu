@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(GT, 7) wah_enc_write(const __grid_constant__ E
   const uint32_t prev = enc_groups<SRC>(S, b, v, s0);
   const uint32_t nv = valid_groups(S, b, t);
   const GroupMasks M = group_masks(v, prev, nv == 32 ? 0xffffffffu : (1u << nv) - 1u, b == 0 && t == 0);
-  const uint64_t at = sum_before<GT>(bcnt, b, scanned);  // 
+  const uint64_t at = sum_before<GT>(bcnt, b, scanned);
   uint32_t total;
   uint32_t pos = block_excl_scan<GT, uint32_t>(__popc(M.start), &total);
   // groups from the end of the thread's to the next start, or to the block's end
