@@ -37,13 +37,15 @@ constexpr uint32_t FT_THREADS = 256;
 constexpr uint32_t FT_WARPS = FT_THREADS / 32;
 
 OpNeeds op_needs(const mb_op &O) {
-  OpNeeds n{0, 0};
+  OpNeeds n{0, 0, false};
   for (uint32_t k = 0; k < O.nkey; ++k) n.kv_mask |= 1u << O.keys[k].src;
   if (O.vkind != MB_V_ONE) n.kv_mask |= 1u << O.va;
   if (O.vkind == MB_V_MUL || O.vkind == MB_V_SUB) n.kv_mask |= 1u << O.vb;
   uint32_t nt = 0;
   for (uint32_t c = 0; c < O.nclause; ++c) nt += O.clause_len[c];
   for (uint32_t t = 0; t < nt; ++t) n.filt_mask |= 1u << O.terms[t].src;
+  for (uint32_t s = 0; s < O.nsrc; ++s)
+    if ((n.kv_mask >> s & 1u) && O.src[s].fk && n.kv_mask != 1u << s) n.behind_key = true;
   return n;
 }
 
@@ -226,17 +228,20 @@ __device__ __forceinline__ void compact_chunk(const mb_op &O, const OpNeeds &N, 
 // 488 -> 344, an OR over 0.5 % 89 -> 88.  From 16 rows a chunk on; 32 and 48 are slower by up to
 // 1.2 and 1.4 times where the chunks of a table lie on both sides (an OR over 6 %, 240M
 // rows: 190 us at 16, 228, 273).
+// Several sources with one behind a foreign key keep drain64: op_eval would wait for the
+// key, its dimension and each of the others in turn (120M rows, nearly all selected, a dimension key, a
+// date and a value: 3,029 us, 3,475).
 // With candidate checks drain64 alone: both in one kernel make the sparse cases 3 to 20 %
 // slower, and op_eval on rows that fail their checks takes up to 1.46 times as long.
 constexpr uint32_t ANY_DENSE = 16;
-template <bool CHK, int GS>
+template <bool CHK, int GS, bool DENSE>
 struct AnyDrain {
   const mb_op &O;
   OpNeeds N;
   uint32_t nr_grp;
   __device__ __forceinline__ void drain(const uint32_t *q, uint32_t n, uint32_t rows, const GrpCtx &G, int64_t &acc,
                                         uint32_t &cnt) const {
-    if (CHK || rows < ANY_DENSE) {
+    if (!DENSE || rows < ANY_DENSE) {
       drain64<CHK ? DR_FLAG : DR_NOCHK, GS>(O, N, q, n, nr_grp, G, acc, cnt);
       return;
     }
@@ -251,15 +256,15 @@ struct AnyDrain {
   }
 };
 
-// Without checks the CTAs an SM are named (64 registers a thread): left alone, the compiler
-// takes 48 for most and spills, sparse programs up to 12 % slower (24M rows, an OR over
-// 0.5 %: 21.8 -> 19.4 us).
-template <int V, bool CHK, int GS, bool CNF>
-__global__ void __launch_bounds__(FW_THREADS, CHK ? 0 : 4)
+// DENSE: dense rows a row a lane (AnyDrain).  Such kernels name the CTAs an SM (64 registers a
+// thread): left alone, the compiler takes 48 for most and spills, sparse programs up to
+// 12 % slower (24M rows, an OR over 0.5 %: 21.8 -> 19.4 us).
+template <int V, bool CHK, int GS, bool CNF, bool DENSE>
+__global__ void __launch_bounds__(FW_THREADS, DENSE ? 4 : 0)
 fused_warp_kernel(const __grid_constant__ DevPrg P, const __grid_constant__ mb_op O, OpNeeds N, uint32_t nr_grp,
                   uint32_t hcap, unsigned long long *__restrict__ out, unsigned long long *__restrict__ nqual) {
   extern __shared__ __align__(128) uint8_t smem[];
-  fused_warp_body<V, CHK, GS, CNF>(P, AnyDrain<CHK, GS>{O, N, nr_grp}, nr_grp, hcap, out, nqual, smem);
+  fused_warp_body<V, CHK, GS, CNF>(P, AnyDrain<CHK, GS, DENSE>{O, N, nr_grp}, nr_grp, hcap, out, nqual, smem);
 }
 
 // T = FT_THREADS * V words per CTA tile.
@@ -451,10 +456,18 @@ static mb_status launch_fw(const DevPrg &P, const mb_op &O, uint32_t nr_grp, uin
     return fw_launch(kern, V, P.nwords, grp_smem_bytes(GS, nr_grp, hcap), warps, cps, st, P, O, op_needs(O), nr_grp,
                      hcap, reinterpret_cast<unsigned long long *>(out), reinterpret_cast<unsigned long long *>(nq));
   };
-  if constexpr (V < 4) {  // (general programs of four words run in the general kernel)
-    if (!P.cnf) return go(fused_warp_kernel<V, CHK, GS, false>);
+  if constexpr (!CHK) {
+    if (!op_needs(O).behind_key) {
+      if constexpr (V < 4) {  // (general programs of four words run in the general kernel)
+        if (!P.cnf) return go(fused_warp_kernel<V, CHK, GS, false, true>);
+      }
+      return go(fused_warp_kernel<V, CHK, GS, true, true>);
+    }
   }
-  return go(fused_warp_kernel<V, CHK, GS, true>);
+  if constexpr (V < 4) {
+    if (!P.cnf) return go(fused_warp_kernel<V, CHK, GS, false, false>);
+  }
+  return go(fused_warp_kernel<V, CHK, GS, true, false>);
 }
 
 template <int V, bool CHK>

@@ -658,15 +658,18 @@ static mb_status scan_rest(uint64_t n, const mb_op &op, uint32_t done, uint32_t 
     if (sh == 2) return scan_shape<2>(C, S, narrow, join, A);
     if (sh == 3) return scan_shape<3>(C, S, narrow, join, A);
   }
-  // An interpreted op goes through the screens where they are its whole filter, or where a
-  // dimension's key bits are among them, on tables of a tile a warp and more.  Else the row
-  // scan is the faster.  Row scan / screens, us, 240M rows, 200 groups (6M, 300K in
+  // An interpreted op goes through the screens where it has one, a range on a fact column or
+  // a dimension's key bits, on tables of a tile a warp and more.  Else the row scan is the
+  // faster.  Row scan / screens, us, 240M rows, 200 groups (6M, 300K in
   // brackets): half of the rows by one range 1,033 / 1,062 (36 / 41, 13 / 22), a tenth
   // 443 / 365 (26 / 18, 11 / 12), two ranges 1,292 / 646 (43 / 29, 12 / 17); no clause 1,398 /
-  // 1,598 (42 / 60, 20 / 32), a dimension's clause 1,073 / 2,790 (39 / 96, 14 / 53), a range and
-  // a dimension's clause 957 / 1,212 (36 / 44, 12 / 26), an OR 1,435 / 2,987 (47 / 108, 14 /
-  // 53); 60M rows, an 8-byte value or clause 272 / 312 and 264 / 326.
-  if (A.ntab == 0 && (nr == 0 || O.nclause || op_reads_wide(op) || n < (uint64_t)dev_info().sms * SC_WARPS * SC_TILE)) {
+  // 1,598 (42 / 60, 20 / 32), a dimension's clause 1,073 / 2,790 (39 / 96, 14 / 53), an OR
+  // 1,435 / 2,987 (47 / 108, 14 / 53); 60M rows, an 8-byte value or clause 272 / 312 and 264 /
+  // 326.  Where clauses are left for the rows that pass the screens, it depends on how many do:
+  // a third and a dimension's clause 957 / 1,230 (36 / 45, 12 / 26); the benchmark's queries
+  // over unindexed dimensions, 120M rows: flight 2 405 / 433, 338 / 312, 305 / 251, flight 3
+  // 565 / 536, 233 / 176, 187 / 122, 173 / 89, flight 4 638 / 755, 544 / 302, 224 / 132.
+  if (A.ntab == 0 && (nr == 0 || op_reads_wide(op) || n < (uint64_t)dev_info().sms * SC_WARPS * SC_TILE)) {
     switch (gs) {
     case GS_SCALAR: return join_gs<GS_SCALAR>(C, op);
     case GS_SHARED: return join_gs<GS_SHARED>(C, op);

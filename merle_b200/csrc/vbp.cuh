@@ -222,9 +222,11 @@ namespace mb {
 // asked for in the launch.
 bool fused_warp_applies(const DevPrg &P, const mb_op &O, size_t grp_bytes, uint32_t warps);
 // Which op sources every row needs (keys, value) and which only uncertain
-// rows need (filter terms).
+// rows need (filter terms); behind_key: a row needs several sources, one of them through a
+// foreign key.
 struct OpNeeds {
   uint32_t kv_mask, filt_mask;
+  bool behind_key;
 };
 OpNeeds op_needs(const mb_op &O);
 // A source the op needs has 8-byte elements.
