@@ -534,19 +534,20 @@ mb_status fused_warp(const DevPrg &P, bool vec4, const mb_op &O, uint32_t sure, 
   const bool compiled = sh >= 0 && (sh == 0 ? gs == GS_SCALAR : gs != GS_SCALAR && nr_grp >= GRP_DIRECT_MIN);
   // Words a lane: wider tiles mean fewer, wider loads and fewer warps at work.
   // Device time in us at V = 1 / 2 / 4: 13 SSB queries, 1M rows 179 / 185 / 189; with a
-  // 24-query spanning and a 24-query random mix beside them (narrow columns):
-  //   30M      322 / 304 / 296     1,027 / 941 / 1,011      526 / 470 / 454
+  // 24-query spanning and a 24-query random mix beside them (narrow columns), back to back:
   //   60M      533 / 477 / 478     1,788 / 1,555 / 1,607    833 / 702 / 693
-  //   90M      741 / 656 / 647     2,547 / 2,186 / 2,193  1,135 / 946 / 896
   //   120M     935 / 827 / 808     3,302 / 2,787 / 2,763  1,426 / 1,159 / 1,090
   //   200M   1,460 / 1,272 / 1,240  5,278 / 4,401 / 4,266  2,144 / 1,727 / 1,619
-  // (at 60M two words win on one mix by 3 % and lose on another by 1 %, at 90M four
-  // lose on none by more than 0.4 %, and beyond that win everywhere).
+  // and V = 2 / 4 with the L2 flushed before each query:
+  //   90M      792 / 786           2,408 / 2,408          1,076 / 1,034
+  //   120M     972 / 968           3,022 / 2,995          1,324 / 1,263
+  //   162M   1,232 / 1,214         3,946 / 3,834          1,677 / 1,584
+  // (at 120M the densest query of the 13 still loses 7 % by four).
   // An interpreted op does not take four: 240M rows, 256 groups, a chain over 6 % of
   // the rows 196 / 189 / 197 us, over a third 640 / 656 / 662, with checks over 6 % 526 / 583
   // / 734 (over 0.1 % it gains 9 %: 79 / 69 / 63); a general program in this kernel, an OR
   // over 30 %, - / 429 / 736, with checks 1,510 / 1,609 / 3,367.
-  if (V == 0) V = P.nrows < 4000000 ? 1 : !compiled || P.nrows < 75000000 ? 2 : 4;
+  if (V == 0) V = P.nrows < 4000000 ? 1 : !compiled || P.nrows < 150000000 ? 2 : 4;
   if (V == 4 && !P.cnf) V = 2;             // (no kernel of four; fused_grpby does not ask for it)
   warps = fw_warps(warps);
   if (!vec4) V = 1;                        // unaligned bitmaps: word loads

@@ -146,11 +146,11 @@ def test_sparse_and_dense_chunks(mb, cuda, instrs, density):
 
 
 def test_templates_on_large_tables_take_four_words_a_lane(mb, cuda):
-    """24 random queries, 120M rows: 1,159 us at two words a lane, 1,090 at four (6 %);
+    """24 random queries, 162M rows: 1,479 us at two words a lane, 1,387 at four (6 %);
     half of that parts them and the scatter of the least of 9 runs."""
     e = Engine(0)
     try:
-        e.gen_star(2, 20, 120_000_000)
+        e.gen_star(2, 27, 162_000_000)
         e.build_index()
         qs = WL.random_mix(3, 24)
         out, nq = D.empty(sum(max(1, e.ngroups(q)) for q in qs), 8), D.empty(len(qs), 8)
